@@ -29,6 +29,7 @@
 #include <type_traits>
 
 #include "rkdg_internal.hpp"
+#include "roots.cuh"
 
 namespace rkdg {
 
@@ -268,12 +269,12 @@ __device__ __forceinline__ void ghost(int tag, const Real u[4], const Real far[4
     }
 }
 
-// Reciprocal, quotient and square root: IEEE in FP64 (the parity path);
-// in FP32 the PTX approximations (rcp.approx, rsqrt.approx: about 1 ulp),
-// which the FP32 precision form's tolerance absorbs, with subnormal inputs
-// and results flushed to zero (.ftz: one instruction each, no subnormal
-// range handling; the arguments are densities, pressures, edge lengths and
-// wave-speed differences, all far above the subnormal range).
+// Reciprocal and square root: within one unit in the last place in FP64
+// (roots.cuh); in FP32 the PTX approximations (rcp.approx, rsqrt.approx:
+// about 1 ulp), which the FP32 precision form's tolerance absorbs, with
+// subnormal inputs and results flushed to zero (.ftz: one instruction each,
+// no subnormal range handling; the arguments are densities, pressures, edge
+// lengths and wave-speed differences, all far above the subnormal range).
 __device__ __forceinline__ float rcp_ftz(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -284,12 +285,16 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-__device__ __forceinline__ double rcp_(double x) { return 1.0 / x; }
+__device__ __forceinline__ double rcp_(double x) { return rcp_f64(x); }
 __device__ __forceinline__ float rcp_(float x) { return rcp_ftz(x); }
-__device__ __forceinline__ double div_(double a, double b) { return a / b; }
-__device__ __forceinline__ float div_(float a, float b) { return a * rcp_ftz(b); }
-__device__ __forceinline__ double sqrt_(double x) { return sqrt(x); }
+__device__ __forceinline__ double sqrt_(double x) { return sqrt_f64(x); }
 __device__ __forceinline__ float sqrt_(float x) { return x * rsqrt_ftz(x); }
+// length and reciprocal length from the squared length: one root for both
+__device__ __forceinline__ void lengths_(double x, double& len, double& inv) { roots_f64(x, len, inv); }
+__device__ __forceinline__ void lengths_(float x, float& len, float& inv) {
+    inv = rsqrt_ftz(x);
+    len = x * inv;
+}
 
 // Normal Euler flux through the scaled normal (Nx, Ny): F Nx + G Ny.
 template <typename Real>
@@ -307,41 +312,38 @@ __device__ __forceinline__ void normal_flux(const Real u[4], Real Nx, Real Ny, R
 
 // HLLC through the unit normal (nx, ny) (Toro, Riemann Solvers and Numerical
 // Methods for Fluid Dynamics, 3rd ed., sec. 10.4): Davis wave-speed bounds
-// (eq. 10.48), contact speed S_M (eq. 10.37), star flux in its pressure form
-// F*_K = (S_M (S_K U_K - F_K) + S_K p* (0, nx, ny, S_M)) / (S_K - S_M),
-// p* = p_K + rho_K (S_K - q_K)(S_M - q_K).  Branch-free: both physical
-// fluxes and the star flux are formed and the result selected (F_L when
-// S_L >= 0, F_R when S_R <= 0), so a warp whose points fall in different
-// wave regions runs one path; a star value formed where it is not selected
-// (even inf or NaN) is discarded.
+// (eq. 10.48), contact speed S_M (eq. 10.37).  Branch-free with one
+// selection: the result is F_K + c (U_K + ex) with K = L when S_L >= 0, R
+// when S_R <= 0 (both with c = 0) and else the side of S_M, where
+//   c (U_K + ex) = S_K (U*_K - U_K),  ex = (0, d_K n, d_K S_M + p_K),
+//   d_K = rho_K (S_K - q_K),  c = S_K (S_M - q_K) / (S_K - S_M),
+// so a warp whose points fall in different wave regions runs one path and
+// only the selected side's physical flux is formed.  The two densities share
+// one reciprocal.
 template <typename Real>
 __device__ __forceinline__ void hllc(const Real uL[4], const Real uR[4], Real nx, Real ny,
                                      Real gamma, Real f[4]) {
     const Real gm1 = gamma - Real(1);
-    Real rL = uL[0], rR = uR[0];
-    Real iL = rcp_(rL), iR = rcp_(rR);
-    Real vxL = uL[1] * iL, vyL = uL[2] * iL, vxR = uR[1] * iR, vyR = uR[2] * iR;
-    Real pL = gm1 * (uL[3] - Real(0.5) * (uL[1] * vxL + uL[2] * vyL));
-    Real pR = gm1 * (uR[3] - Real(0.5) * (uR[1] * vxR + uR[2] * vyR));
-    Real qL = vxL * nx + vyL * ny, qR = vxR * nx + vyR * ny;
-    Real cL = sqrt_(gamma * pL * iL), cR = sqrt_(gamma * pR * iR);
-    Real SL = fmin(qL - cL, qR - cR), SR = fmax(qL + cL, qR + cR);
-    const Real FL[4] = {rL * qL, uL[1] * qL + pL * nx, uL[2] * qL + pL * ny, (uL[3] + pL) * qL};
-    const Real FR[4] = {rR * qR, uR[1] * qR + pR * nx, uR[2] * qR + pR * ny, (uR[3] + pR) * qR};
-    Real dL = rL * (SL - qL), dR = rR * (SR - qR);
-    Real SM = div_(pR - pL + dL * qL - dR * qR, dL - dR);
-    const bool left = SM >= Real(0);
-    Real d = left ? dL : dR, p = left ? pL : pR, q = left ? qL : qR, S = left ? SL : SR;
-    Real ps = p + d * (SM - q);
-    Real k = rcp_(S - SM);
+    const Real irr = rcp_(uL[0] * uR[0]);
+    const Real iL = uR[0] * irr, iR = uL[0] * irr;
+    const Real vxL = uL[1] * iL, vyL = uL[2] * iL, vxR = uR[1] * iR, vyR = uR[2] * iR;
+    const Real pL = gm1 * (uL[3] - Real(0.5) * (uL[1] * vxL + uL[2] * vyL));
+    const Real pR = gm1 * (uR[3] - Real(0.5) * (uR[1] * vxR + uR[2] * vyR));
+    const Real qL = vxL * nx + vyL * ny, qR = vxR * nx + vyR * ny;
+    const Real cL = sqrt_(gamma * pL * iL), cR = sqrt_(gamma * pR * iR);
+    const Real SL = fmin(qL - cL, qR - cR), SR = fmax(qL + cL, qR + cR);
+    const Real dL = uL[0] * (SL - qL), dR = uR[0] * (SR - qR);
+    const Real SM = (pR - pL + dL * qL - dR * qR) * rcp_(dL - dR);
     const bool sl = SL >= Real(0), sr = SR <= Real(0);
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-        const Real uK = left ? uL[v] : uR[v], FK = left ? FL[v] : FR[v];
-        const Real pn = v == 0 ? Real(0) : (v == 1 ? nx : (v == 2 ? ny : SM));
-        const Real fs = (SM * (S * uK - FK) + S * ps * pn) * k;
-        f[v] = sl ? FL[v] : (sr ? FR[v] : fs);
-    }
+    const bool left = sl || (!sr && SM >= Real(0));
+    const Real d = left ? dL : dR, p = left ? pL : pR, q = left ? qL : qR, S = left ? SL : SR;
+    const Real u0 = left ? uL[0] : uR[0], u1 = left ? uL[1] : uR[1], u2 = left ? uL[2] : uR[2],
+               u3 = left ? uL[3] : uR[3];
+    const Real c = (sl || sr) ? Real(0) : S * (SM - q) * rcp_(S - SM);
+    f[0] = u0 * q + c * u0;
+    f[1] = (u1 * q + p * nx) + c * (u1 + d * nx);
+    f[2] = (u2 * q + p * ny) + c * (u2 + d * ny);
+    f[3] = (u3 + p) * q + c * ((u3 + p) + d * SM);
 }
 
 // ------------------------------------------- deviation form (FP32 path) --

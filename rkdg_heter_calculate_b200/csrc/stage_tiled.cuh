@@ -495,16 +495,14 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
                 dev_flux(w, pw, rs, j00, j01, fx);
                 dev_flux(w, pw, rs, j10, j11, fy);
             } else {
-                Real ri = rcp_(w[0]);
-                Real vx = w[1] * ri, vy = w[2] * ri;
-                Real p = gm1 * (w[3] - Real(0.5) * (w[1] * vx + w[2] * vy));
-                Real F[4] = {w[1], w[1] * vx + p, w[2] * vx, (w[3] + p) * vx};
-                Real G[4] = {w[2], w[1] * vy, w[2] * vy + p, (w[3] + p) * vy};
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    fx[v] = j00 * F[v] + j01 * G[v];
-                    fy[v] = j10 * F[v] + j11 * G[v];
-                }
+                // the fluxes through the rows of 2 area J^-1, by their
+                // contravariant speeds
+                const Real ri = rcp_(w[0]);
+                const Real vx = w[1] * ri, vy = w[2] * ri;
+                const Real p = gm1 * (w[3] - Real(0.5) * (w[1] * vx + w[2] * vy));
+                const Real q0 = j00 * vx + j01 * vy, q1 = j10 * vx + j11 * vy, h = w[3] + p;
+                fx[0] = w[0] * q0, fx[1] = w[1] * q0 + j00 * p, fx[2] = w[2] * q0 + j01 * p, fx[3] = h * q0;
+                fy[0] = w[0] * q1, fy[1] = w[1] * q1 + j10 * p, fy[2] = w[2] * q1 + j11 * p, fy[3] = h * q1;
             }
             if constexpr (PK) {
                 acc_rows<1, NB>(R, fx, t2.vdxi[q]);
@@ -614,8 +612,8 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
             const int kind = c & 3, se = (c >> 2) & 3, idx = c >> 4;
             // physical normal N (|N| = edge length) and unit normal of edge k
             const Real Nx = s_nrm[(NC * k + 0) * BT + le], Ny = s_nrm[(NC * k + 1) * BT + le];
-            const Real len = sqrt_(Nx * Nx + Ny * Ny);
-            const Real il = rcp_(len);
+            Real len, il;
+            lengths_(Nx * Nx + Ny * Ny, len, il);
             const Real nx = Nx * il, ny = Ny * il;
             Real mL[4], mR[4];
             if constexpr (MEANS) {
