@@ -35,6 +35,7 @@ struct rkdg_batch {
     uint16_t* task = nullptr;
     int32_t* perm = nullptr;
     double* far = nullptr;
+    float* ref32 = nullptr;  // [S][8] the FP32 kernels' reference states
     double* staging = nullptr;
     StepCtl* ctl = nullptr;
     StepCtl* h_ctl = nullptr;
@@ -135,6 +136,7 @@ StageArgs stage_args(const rkdg_batch* b) {
     a.gamma = b->p.gamma;
     for (int v = 0; v < 4; ++v) a.far[v] = b->p.farfield[v];
     a.far_sid = b->far;
+    a.ref32 = b->ref32;
     a.lo_row = lo_row(b);
     return a;
 }
@@ -270,7 +272,7 @@ void destroy_batch(rkdg_batch* b) {
     if (b->stream) cudaStreamSynchronize(b->stream);
     for (void* p : {b->U[0], b->U[1], b->U[2]}) cudaFree(p);
     for (void* p : {(void*)b->jinv, (void*)b->tcode, (void*)b->tdesc, (void*)b->halo, (void*)b->task,
-                    (void*)b->perm, (void*)b->far, (void*)b->staging, (void*)b->ctl})
+                    (void*)b->perm, (void*)b->far, (void*)b->ref32, (void*)b->staging, (void*)b->ctl})
         cudaFree(p);
     if (b->h_ctl) cudaFreeHost(b->h_ctl);
     if (b->ev_fork) cudaEventDestroy(b->ev_fork);
@@ -386,6 +388,10 @@ int rkdg_batch_create(int32_t nsolves, const rkdg_mesh_desc* meshes, const int32
         b->far = (double*)balloc(b, sizeof(double) * far.size());
         h2d(b, b->far, far);
         b->far_host = far;
+        std::vector<float> ref((size_t)8 * nsolves);
+        for (int s = 0; s < nsolves; ++s) ref_state32(&far[4 * s], p.gamma, &ref[8 * s]);
+        b->ref32 = (float*)balloc(b, sizeof(float) * ref.size());
+        h2d(b, b->ref32, ref);
         b->staging = (double*)balloc(b, sizeof(double) * 24 * (size_t)maxT);
         b->ctl = (StepCtl*)balloc(b, sizeof(StepCtl) * nsolves);
         for (int s = 0; s < nsolves; ++s) b->h_ctl[s].cfl = p.cfl;

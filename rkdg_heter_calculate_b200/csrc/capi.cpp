@@ -166,6 +166,7 @@ StageArgs base_args(const rkdg_ctx* c) {
     a.ctl = c->d.ctl;
     a.gamma = c->p.gamma;
     for (int v = 0; v < 4; ++v) a.far[v] = c->p.farfield[v];
+    a.ref32 = c->d.ref32;
     a.lo_row = lo_row(c);
     a.tvb_m = c->p.tvb_m;
     return a;
@@ -302,6 +303,7 @@ void destroy_ctx(rkdg_ctx* c) {
     cudaFree(c->d.partial);
     cudaFree(c->d.ctl);
     cudaFree(c->d.far);
+    cudaFree(c->d.ref32);
     cudaFree(c->d.tcode);
     cudaFree(c->d.tdesc);
     cudaFree(c->d.halo);
@@ -470,6 +472,10 @@ int create_ctx(const rkdg_mesh_desc* mesh, const rkdg_params* params, int32_t n_
         c->d.far = (double*)dev_alloc(c, sizeof(double) * 4);
         RKDG_CUDA_TRY(cudaMemcpyAsync(c->d.far, params->farfield, sizeof(double) * 4,
                                       cudaMemcpyHostToDevice, c->stream));
+        float ref[8];
+        ref_state32(params->farfield, params->gamma, ref);
+        c->d.ref32 = (float*)dev_alloc(c, sizeof(ref));
+        RKDG_CUDA_TRY(cudaMemcpyAsync(c->d.ref32, ref, sizeof(ref), cudaMemcpyHostToDevice, c->stream));
         c->h_ctl->cfl = params->cfl;
         push_ctl(c);
         sync(c);

@@ -61,6 +61,12 @@ struct Tab2 {
     float2 nephiw[3][kMaxNG][kMaxNB];
 };
 __constant__ Tab2 c_tab_f2[kNumCfg];
+// The edge tables in global memory, [3][NG][NB] packed per configuration: a
+// CTA copies its configuration's into shared memory with coalesced loads
+// (through the constant bank each lane's own address is a replay, which with
+// the FP64 reference state per thread cost the FP32 P2 stage 5 %).
+__device__ float2 g_ephi_f2[kNumCfg][3 * kMaxNG * kMaxNB];
+__device__ double g_ephi_d[kNumCfg][3 * kMaxNG * kMaxNB];
 
 // Two-lane FP32 arithmetic (PTX fma/mul/add/sub .f32x2, sm_100a): each lane is
 // one IEEE single-precision operation (a fused multiply-add rounds once).
@@ -112,16 +118,16 @@ __device__ __forceinline__ const Tab<float>& tab<float>(int c) { return c_tab_f[
 
 void upload_tables(int nq, int ng) {
     RuleTables t = make_tables(nq, ng);
-    // the tile kernel forms the psi_0 term once (psi_0 is the same constant
-    // at every volume and edge point) and skips the eta-derivative of psi_1
-    // (a function of xi alone): both hold exactly for the native basis
+    // the stage kernels take psi_0 as one at every volume and edge point and
+    // skip the eta-derivative of psi_1 (a function of xi alone): both hold
+    // exactly for the native basis
     for (int q = 0; q < nq; ++q)
-        if (t.vphi[q][0] != t.vphi[0][0] || t.veta_w[q][1] != 0.0)
-            throw Error{RKDG_ERR_INVALID, "basis tables: psi_0 not constant or psi_1 not a function of xi"};
+        if (t.vphi[q][0] != 1.0 || t.veta_w[q][1] != 0.0)
+            throw Error{RKDG_ERR_INVALID, "basis tables: psi_0 not one or psi_1 not a function of xi"};
     for (int k = 0; k < 3; ++k)
         for (int g = 0; g < ng; ++g)
-            if (t.ephi[k][g][0] != t.vphi[0][0])
-                throw Error{RKDG_ERR_INVALID, "basis tables: psi_0 not constant on the edges"};
+            if (t.ephi[k][g][0] != 1.0)
+                throw Error{RKDG_ERR_INVALID, "basis tables: psi_0 not one on the edges"};
     Tab<double> d{};
     Tab<float> f{};
     for (int q = 0; q < kMaxNQ; ++q)
@@ -170,6 +176,17 @@ void upload_tables(int nq, int ng) {
     RKDG_CUDA_TRY(cudaMemcpyToSymbol(c_tab_d, &d, sizeof(d), sizeof(d) * c));
     RKDG_CUDA_TRY(cudaMemcpyToSymbol(c_tab_f, &f, sizeof(f), sizeof(f) * c));
     RKDG_CUDA_TRY(cudaMemcpyToSymbol(c_tab_f2, &f2, sizeof(f2), sizeof(f2) * c));
+    const int nb = ng == 2 ? 3 : 6;  // P1 and P2 edge rules
+    float2 ef[3 * kMaxNG * kMaxNB] = {};
+    double ed[3 * kMaxNG * kMaxNB] = {};
+    for (int k = 0; k < 3; ++k)
+        for (int g = 0; g < ng; ++g)
+            for (int i = 0; i < nb; ++i) {
+                ef[(k * ng + g) * nb + i] = dup(t.ephi[k][g][i]);
+                ed[(k * ng + g) * nb + i] = t.ephi[k][g][i];
+            }
+    RKDG_CUDA_TRY(cudaMemcpyToSymbol(g_ephi_f2, ef, sizeof(ef), sizeof(ef) * c));
+    RKDG_CUDA_TRY(cudaMemcpyToSymbol(g_ephi_d, ed, sizeof(ed), sizeof(ed) * c));
 }
 
 // --------------------------------------------------------- state packs --
@@ -251,24 +268,6 @@ __device__ __forceinline__ void store_rows(Real* __restrict__ U, int ld, int e, 
 }
 
 // ------------------------------------------------------------- physics --
-// Ghost state of a boundary edge (the reference's boundaryCondition kernel,
-// src/kernelfunctions.cu:184-268, applied inline): 1 far field, 2 outflow
-// copy, 3 slip wall mirroring the momentum about the unit normal.
-template <typename Real>
-__device__ __forceinline__ void ghost(int tag, const Real u[4], const Real far[4], Real nx, Real ny,
-                                      Real g[4]) {
-    if (tag == RKDG_BC_FARFIELD) {
-        g[0] = far[0], g[1] = far[1], g[2] = far[2], g[3] = far[3];
-    } else if (tag == RKDG_BC_OUTFLOW) {
-        g[0] = u[0], g[1] = u[1], g[2] = u[2], g[3] = u[3];
-    } else {
-        g[0] = u[0];
-        g[3] = u[3];
-        g[1] = u[1] * (ny * ny - nx * nx) - Real(2) * nx * ny * u[2];
-        g[2] = u[2] * (nx * nx - ny * ny) - Real(2) * nx * ny * u[1];
-    }
-}
-
 // Reciprocal and square root: within one unit in the last place in FP64
 // (roots.cuh); in FP32 the PTX approximations (rcp.approx, rsqrt.approx:
 // about 1 ulp), which the FP32 precision form's tolerance absorbs, with
@@ -289,6 +288,12 @@ __device__ __forceinline__ double rcp_(double x) { return rcp_f64(x); }
 __device__ __forceinline__ float rcp_(float x) { return rcp_ftz(x); }
 __device__ __forceinline__ double sqrt_(double x) { return sqrt_f64(x); }
 __device__ __forceinline__ float sqrt_(float x) { return x * rsqrt_ftz(x); }
+// Operations that the compiler may not contract with their neighbours: a sum
+// of products written with them and fma rounds alike in every kernel.
+__device__ __forceinline__ double add_(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float add_(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double mul_(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_(float a, float b) { return __fmul_rn(a, b); }
 // length and reciprocal length from the squared length: one root for both
 __device__ __forceinline__ void lengths_(double x, double& len, double& inv) { roots_f64(x, len, inv); }
 __device__ __forceinline__ void lengths_(float x, float& len, float& inv) {
@@ -296,54 +301,23 @@ __device__ __forceinline__ void lengths_(float x, float& len, float& inv) {
     len = x * inv;
 }
 
-// Normal Euler flux through the scaled normal (Nx, Ny): F Nx + G Ny.
+// Ghost state of a boundary edge (the reference's boundaryCondition kernel,
+// src/kernelfunctions.cu:184-268, applied inline): 1 far field, 2 outflow
+// copy, 3 slip wall mirroring the momentum about the unit normal.
 template <typename Real>
-__device__ __forceinline__ void normal_flux(const Real u[4], Real Nx, Real Ny, Real gm1, Real f[4],
-                                            Real& p) {
-    Real ri = rcp_(u[0]);
-    Real vx = u[1] * ri, vy = u[2] * ri;
-    p = gm1 * (u[3] - Real(0.5) * (u[1] * vx + u[2] * vy));
-    Real qn = vx * Nx + vy * Ny;
-    f[0] = u[0] * qn;
-    f[1] = u[1] * qn + p * Nx;
-    f[2] = u[2] * qn + p * Ny;
-    f[3] = (u[3] + p) * qn;
-}
-
-// HLLC through the unit normal (nx, ny) (Toro, Riemann Solvers and Numerical
-// Methods for Fluid Dynamics, 3rd ed., sec. 10.4): Davis wave-speed bounds
-// (eq. 10.48), contact speed S_M (eq. 10.37).  Branch-free with one
-// selection: the result is F_K + c (U_K + ex) with K = L when S_L >= 0, R
-// when S_R <= 0 (both with c = 0) and else the side of S_M, where
-//   c (U_K + ex) = S_K (U*_K - U_K),  ex = (0, d_K n, d_K S_M + p_K),
-//   d_K = rho_K (S_K - q_K),  c = S_K (S_M - q_K) / (S_K - S_M),
-// so a warp whose points fall in different wave regions runs one path and
-// only the selected side's physical flux is formed.  The two densities share
-// one reciprocal.
-template <typename Real>
-__device__ __forceinline__ void hllc(const Real uL[4], const Real uR[4], Real nx, Real ny,
-                                     Real gamma, Real f[4]) {
-    const Real gm1 = gamma - Real(1);
-    const Real irr = rcp_(uL[0] * uR[0]);
-    const Real iL = uR[0] * irr, iR = uL[0] * irr;
-    const Real vxL = uL[1] * iL, vyL = uL[2] * iL, vxR = uR[1] * iR, vyR = uR[2] * iR;
-    const Real pL = gm1 * (uL[3] - Real(0.5) * (uL[1] * vxL + uL[2] * vyL));
-    const Real pR = gm1 * (uR[3] - Real(0.5) * (uR[1] * vxR + uR[2] * vyR));
-    const Real qL = vxL * nx + vyL * ny, qR = vxR * nx + vyR * ny;
-    const Real cL = sqrt_(gamma * pL * iL), cR = sqrt_(gamma * pR * iR);
-    const Real SL = fmin(qL - cL, qR - cR), SR = fmax(qL + cL, qR + cR);
-    const Real dL = uL[0] * (SL - qL), dR = uR[0] * (SR - qR);
-    const Real SM = (pR - pL + dL * qL - dR * qR) * rcp_(dL - dR);
-    const bool sl = SL >= Real(0), sr = SR <= Real(0);
-    const bool left = sl || (!sr && SM >= Real(0));
-    const Real d = left ? dL : dR, p = left ? pL : pR, q = left ? qL : qR, S = left ? SL : SR;
-    const Real u0 = left ? uL[0] : uR[0], u1 = left ? uL[1] : uR[1], u2 = left ? uL[2] : uR[2],
-               u3 = left ? uL[3] : uR[3];
-    const Real c = (sl || sr) ? Real(0) : S * (SM - q) * rcp_(S - SM);
-    f[0] = u0 * q + c * u0;
-    f[1] = (u1 * q + p * nx) + c * (u1 + d * nx);
-    f[2] = (u2 * q + p * ny) + c * (u2 + d * ny);
-    f[3] = (u3 + p) * q + c * ((u3 + p) + d * SM);
+__device__ __forceinline__ void ghost(int tag, const Real u[4], const Real far[4], Real nx, Real ny,
+                                      Real g[4]) {
+    if (tag == RKDG_BC_FARFIELD) {
+        g[0] = far[0], g[1] = far[1], g[2] = far[2], g[3] = far[3];
+    } else if (tag == RKDG_BC_OUTFLOW) {
+        g[0] = u[0], g[1] = u[1], g[2] = u[2], g[3] = u[3];
+    } else {
+        const Real c = fma(ny, ny, -mul_(nx, nx)), d = mul_(Real(2), mul_(nx, ny));
+        g[0] = u[0];
+        g[3] = u[3];
+        g[1] = fma(u[1], c, -mul_(d, u[2]));
+        g[2] = fma(-u[2], c, -mul_(d, u[1]));
+    }
 }
 
 // ------------------------------------------- deviation form (FP32 path) --
@@ -359,12 +333,11 @@ template <typename Real>
 struct RefState {
     Real rho, mx, my, E, u, v, p, Ep;  // Ep = E + p
 };
-template <typename Real>
-__device__ __forceinline__ RefState<Real> ref_state(const double f[4], double gamma) {
-    const double u = f[1] / f[0], v = f[2] / f[0];
-    const double p = (gamma - 1.0) * (f[3] - 0.5 * (f[1] * u + f[2] * v));
-    return RefState<Real>{(Real)f[0], (Real)f[1], (Real)f[2], (Real)f[3], (Real)u, (Real)v, (Real)p,
-                          (Real)(f[3] + p)};
+// of solve sid, from the table formed on the host (ref_state32)
+__device__ __forceinline__ RefState<float> ref_state(const float* tab, int sid) {
+    const float4* t = reinterpret_cast<const float4*>(tab) + 2 * sid;
+    const float4 a = __ldg(t), b = __ldg(t + 1);
+    return RefState<float>{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 }
 template <typename Real>
 struct DevPrims {
@@ -534,11 +507,11 @@ template <typename Real>
 __device__ __forceinline__ double wave_of(const Real m[4], Real gamma, const Real len[3], Real inv_area,
                                           bool& bad) {
     const Real ri = rcp_(m[0]);
-    const Real u = m[1] * ri, v = m[2] * ri;
-    const Real p = (gamma - Real(1)) * (m[3] - Real(0.5) * (m[1] * u + m[2] * v));
+    const Real u = mul_(m[1], ri), v = mul_(m[2], ri);
+    const Real p = mul_(add_(gamma, Real(-1)), fma(Real(-0.5), fma(m[1], u, mul_(m[2], v)), m[3]));
     bad = !(m[0] > Real(0)) || !(p > Real(0));
-    const Real c = sqrt0_(gamma * p * ri);
-    const Real w = (sqrt0_(u * u + v * v) + c) * ((len[0] + len[1] + len[2]) * inv_area);
+    const Real c = sqrt0_(mul_(mul_(gamma, p), ri));
+    const Real w = mul_(add_(sqrt0_(fma(u, u, mul_(v, v))), c), mul_(add_(add_(len[0], len[1]), len[2]), inv_area));
     return bad ? __longlong_as_double(0x7ff8000000000000LL) : (double)w;
 }
 
@@ -589,6 +562,7 @@ __device__ __forceinline__ void tvb_geometry(Real c0x, Real c0y, Real c1x, Real 
     }
 }
 #include "stage_tiled.cuh"
+#include "stage_fp64.cuh"
 
 // CFL measure of the current state per solve (first step, rkdg_compute_dt):
 // one CTA per tile (its threads loop over the tile's elements), a block max
@@ -1100,6 +1074,12 @@ namespace {
 // Shared-memory attributes of one instantiation for a halo size; returns the
 // dynamic shared memory per CTA.
 
+// The stage kernel of an arithmetic type.
+template <typename Real, int NQ2, int FLUX, int MODE, int ORD, int BT, int LAT = 0>
+constexpr auto stage_kernel() {
+    if constexpr (sizeof(Real) == 8) return &stage_fp64_kernel<NQ2, FLUX, MODE, ORD, BT, LAT>;
+    else return &tiled_stage_kernel<NQ2, FLUX, MODE, ORD, BT>;
+}
 template <typename Real, int NQ2, int FLUX, int MODE, int ORD, int BT, int LAT = 0>
 size_t prepare_tiled(int max_halo) {
     const size_t smem = TiledSmem<Real, ORD, FLUX, BT>::bytes(max_halo);
@@ -1108,16 +1088,15 @@ size_t prepare_tiled(int max_halo) {
                                           std::to_string(max_halo) + " entries need " + std::to_string(smem) +
                                           " bytes of shared memory per CTA, above the device's limit: use "
                                           "128-element tiles or the locality order"};
+    constexpr auto kernel = stage_kernel<Real, NQ2, FLUX, MODE, ORD, BT, LAT>();
     // dynamic + static shared memory above 48 KB needs the opt-in.  Per
     // instantiation; raised when a context with a larger halo appears.
     static size_t configured = 0;
     if (configured == 0)  // give shared memory the whole carveout
-        RKDG_CUDA_TRY(cudaFuncSetAttribute(tiled_stage_kernel<Real, NQ2, FLUX, MODE, ORD, BT, LAT>,
-                                           cudaFuncAttributePreferredSharedMemoryCarveout,
+        RKDG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                            (int)cudaSharedmemCarveoutMaxShared));
     if (smem > configured) {
-        RKDG_CUDA_TRY(cudaFuncSetAttribute(tiled_stage_kernel<Real, NQ2, FLUX, MODE, ORD, BT, LAT>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        RKDG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         configured = smem;
     }
     return smem;
@@ -1126,9 +1105,13 @@ size_t prepare_tiled(int max_halo) {
 template <typename Real, int NQ2, int FLUX, int MODE, int ORD, int BT>
 int occupancy_tiled(int max_halo) {
     const size_t smem = prepare_tiled<Real, NQ2, FLUX, MODE, ORD, BT>(max_halo);
-    int n = 0;
-    RKDG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &n, tiled_stage_kernel<Real, NQ2, FLUX, MODE, ORD, BT>, BT, smem));
+    thread_local size_t of = 0;  // the last answer, per instantiation and thread
+    thread_local int n = 0;
+    if (of != smem) {
+        constexpr auto kernel = stage_kernel<Real, NQ2, FLUX, MODE, ORD, BT>();
+        RKDG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, BT, smem));
+        of = smem;
+    }
     return n;
 }
 
@@ -1136,7 +1119,11 @@ template <typename Real, int NQ2, int FLUX, int MODE, int ORD, int BT, int LAT =
 void launch_tiled(const StageArgs& a, const TileArgs& t, int ctas, cudaStream_t s) {
     const size_t smem = prepare_tiled<Real, NQ2, FLUX, MODE, ORD, BT, LAT>(t.max_halo);
     const int grid = (ctas > 0 && ctas < t.ntiles) ? ctas : t.ntiles;
-    if (grid > 0) tiled_stage_kernel<Real, NQ2, FLUX, MODE, ORD, BT, LAT><<<grid, BT, smem, s>>>(a, t);
+    constexpr auto kernel = stage_kernel<Real, NQ2, FLUX, MODE, ORD, BT, LAT>();
+    TileArgs ta = t;
+    if constexpr (sizeof(Real) == 4)  // FP32 kernels prefetch a device of CTAs ahead (prefetch_ahead)
+        if (grid == t.ntiles) ta.ahead = sm_count() * occupancy_tiled<Real, NQ2, FLUX, MODE, ORD, BT>(t.max_halo);
+    if (grid > 0) kernel<<<grid, BT, smem, s>>>(a, ta);
 }
 
 // Tile sizes the stage kernel is built for: 128 everywhere, 256 for the
@@ -1148,7 +1135,7 @@ template <typename Real, int NQ2, int FLUX, int MODE, int ORD>
 void launch_tiled_bt(const StageArgs& a, const TileArgs& t, int ctas, cudaStream_t s) {
     if (t.tile == 128) {
         if constexpr (sizeof(Real) == 8) {
-            const int fit = sm_count() * TiledOccupancy<Real, ORD, 128, 1>::value;
+            const int fit = sm_count() * Fp64Occupancy<ORD, 128, 1>::value;
             if ((ctas <= 0 || ctas >= t.ntiles) && t.ntiles_dev == nullptr && t.ntiles <= fit)
                 return launch_tiled<Real, NQ2, FLUX, MODE, ORD, 128, 1>(a, t, ctas, s);
         }

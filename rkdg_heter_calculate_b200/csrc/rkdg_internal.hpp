@@ -160,6 +160,15 @@ inline void throw_ctl_error(int error, const std::string& who) {
     if (error) throw Error{RKDG_ERR_STATE, who + ": non-physical state (NaN or non-positive density/pressure)"};
 }
 
+// The FP32 kernels' reference state of a solve from its far-field state:
+// rho, rho u, rho v, E, u, v, p, E + p, formed in FP64 and rounded.
+inline void ref_state32(const double far[4], double gamma, float out[8]) {
+    const double u = far[1] / far[0], v = far[2] / far[0];
+    const double p = (gamma - 1.0) * (far[3] - 0.5 * (far[1] * u + far[2] * v));
+    for (int i = 0; i < 4; ++i) out[i] = (float)far[i];
+    out[4] = (float)u, out[5] = (float)v, out[6] = (float)p, out[7] = (float)(far[3] + p);
+}
+
 struct DeviceArrays {
     void* U[3] = {nullptr, nullptr, nullptr};  // state buffers (A holds U^n)
     double* jinv = nullptr;     // [2][ld][2]
@@ -174,6 +183,7 @@ struct DeviceArrays {
     double* partial = nullptr;  // block partial sums for deterministic totals
     StepCtl* ctl = nullptr;
     double* far = nullptr;      // [4] far-field / reference state (device copy)
+    float* ref32 = nullptr;     // [8] the FP32 kernels' form of it
     // tile tables
     int4* tcode = nullptr;
     int4* tdesc = nullptr;
@@ -199,6 +209,7 @@ struct TileArgs {
     int ntiles;
     const int* ntiles_dev;  // when set, kernels read the tile count here (graph-stable)
     int tile = kTile;       // elements per tile (threads per CTA of the stage kernel): 128 or 256
+    int ahead = 0;          // CTAs of a full device: how far ahead one CTA per tile prefetches (set by the launcher)
 };
 
 struct StageArgs {
@@ -213,6 +224,7 @@ struct StageArgs {
     double gamma;
     double far[4];
     const double* far_sid;  // per-solve far-field states [solves][4], or nullptr
+    const float* ref32;     // FP32: per-solve reference states [solves][8] (ref_state32)
     int last_stage;      // compute wave max / error (and the monitor when asked) in the epilogue
     int monitor;         // last stage: also form the residual monitor max |d mean| (rho, rhoE)
     int lo_row;          // RKDG_FP32C: state row of the cell means' low parts (in U, U0, Unew), else -1

@@ -137,6 +137,7 @@ struct rkdg_server {
     int* ntiles_dev = nullptr;   // [kLists]: active tiles of each list
     StepCtl* ctl = nullptr;
     double* far = nullptr;
+    float* ref32 = nullptr;  // [slots][8] the FP32 kernels' reference states
     int* flags = nullptr;
     int* tile_flags = nullptr;   // [kLists][tcap] the stage kernel's per-tile limiter test, per list
     int* tile_list = nullptr;    // [kLists][kListHead + tcap] the tiles each list's limiter visits
@@ -234,6 +235,7 @@ void enqueue_step(rkdg_server* s) {
         a.gamma = s->p.gamma;
         for (int v = 0; v < 4; ++v) a.far[v] = s->p.farfield[v];
         a.far_sid = s->far;
+        a.ref32 = s->ref32;
         coeffs(s->p.rk, st, a.a, a.b);
         a.U = s->U[pl[0]];
         a.U0 = st == 0 ? nullptr : s->U[pl[1]];
@@ -302,6 +304,9 @@ void upload(rkdg_server* s, Request& r) {
     c.t_final = r.t_final > 0 ? r.t_final : 1e-300;
     h2d(s, s->ctl + r.slot, &c, 1);
     h2d(s, s->far + 4 * r.slot, r.far, 4);
+    float ref[8];
+    ref_state32(r.far, s->p.gamma, ref);
+    h2d(s, s->ref32 + 8 * r.slot, ref, 8);
     int flag = r.limiter ? 1 : 0;
     h2d(s, s->flags + r.slot, &flag, 1);
     RKDG_CUDA_TRY(cudaStreamSynchronize(s->stream));  // host buffers above are temporaries
@@ -512,7 +517,7 @@ void destroy_server(rkdg_server* s) {
     if (s->graph) cudaGraphExecDestroy(s->graph);
     for (void* p : {s->U[0], s->U[1], s->U[2], (void*)s->jinv, (void*)s->tcode, (void*)s->conn, (void*)s->lim,
                     (void*)s->perm, (void*)s->halo, (void*)s->task, (void*)s->desc, (void*)s->ntiles_dev,
-                    (void*)s->ctl, (void*)s->far, (void*)s->flags, (void*)s->tile_flags, (void*)s->tile_list,
+                    (void*)s->ctl, (void*)s->far, (void*)s->ref32, (void*)s->flags, (void*)s->tile_flags, (void*)s->tile_list,
                     (void*)s->staging})
         cudaFree(p);
     if (s->h_ctl) cudaFreeHost(s->h_ctl);
@@ -613,6 +618,10 @@ int rkdg_server_create(const rkdg_params* params, size_t budget, int32_t max_slo
         for (int i = 0; i < max_slots; ++i)
             for (int v = 0; v < 4; ++v) f[4 * i + v] = p.farfield[v];
         h2d(s, s->far, f.data(), f.size());
+        std::vector<float> f32(8 * (size_t)max_slots);
+        for (int i = 0; i < max_slots; ++i) ref_state32(&f[4 * i], p.gamma, &f32[8 * i]);
+        s->ref32 = (float*)salloc(s, sizeof(float) * f32.size());
+        h2d(s, s->ref32, f32.data(), f32.size());
         s->flags = (int*)salloc(s, sizeof(int) * max_slots);
         s->tile_flags = (int*)salloc(s, sizeof(int) * kLists * (size_t)s->tcap);
         s->tile_list = (int*)salloc(s, sizeof(int) * kLists * (kListHead + (size_t)s->tcap));

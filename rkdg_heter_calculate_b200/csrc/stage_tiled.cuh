@@ -1,4 +1,5 @@
-// Tile-staged fused stage kernel (included by kernels.cu).
+// Tile-staged fused stage kernel (included by kernels.cu): the staging
+// pipeline and the FP32 kernel (FP64: stage_pair.cuh).
 //
 // A tile is up to BT consecutive (locality-ordered) elements of one
 // solve; its descriptor names the element range, the solve, the polynomial
@@ -21,6 +22,14 @@
 // its own dt, CFL measure and monitor.  A tile's arithmetic depends only on
 // its own solve's data: results are deterministic and identical whether a
 // solve runs alone or in a batch.
+//
+// What bounds it: the instructions of 24 (P1: 32) warps per SM and, at the
+// start of a CTA, the chain descriptor -> geometry, codes and lists -> state
+// (a quarter of a tile's 20,000 cycles on 500,000 triangles).  So every load
+// that needs no other is issued first, nobody waits for the thread that
+// issues the copies, the reference state comes from a table, and the edge
+// tables are loaded once per CTA: 980,000 P2 triangles 0.288 -> 0.263 ms per
+// step in FP32 and 0.310 -> 0.289 in FP32C, P1 with LLF 0.171 -> 0.158.
 //
 // Staging pipeline: a tile's own state rows are contiguous 16-byte rows in
 // HBM (pack p of element e at (p ld + e) 16), so one thread moves them into
@@ -132,9 +141,9 @@ __device__ __forceinline__ void get4(const Vec4<Real>* p, Real a[4]) {
     const Vec4<Real> t = *p;
     a[0] = t.x, a[1] = t.y, a[2] = t.z, a[3] = t.w;
 }
-// Per-element linear algebra on 4-vectors (the conservative components).
-// FP32 runs it in lane pairs (components 0-1 and 2-3) with the f32x2
-// helpers and the paired tables; FP64 runs the scalar form.  (Pairing the
+// Per-element linear algebra on 4-vectors (the conservative components), in
+// lane pairs (components 0-1 and 2-3) with the f32x2 helpers and the paired
+// tables.  (Pairing the
 // two sides of the HLLC flux the same way executed fewer instructions but
 // more register moves and ran slower.)
 __device__ __forceinline__ float2 lo2(const float a[4]) { return make_float2(a[0], a[1]); }
@@ -186,20 +195,15 @@ struct TiledSmem {
     __host__ __device__ static constexpr size_t bytes(int hm) { return stage_offset(hm) + stage_rows(hm) * 16; }
 };
 
-// Resident CTAs per SM the register allocation is held to: in FP32 24 warps
-// per SM for kernels with P2 tiles (80 registers; 128-element tiles at most
-// 37 KB of shared memory per CTA) and 32 for P1-only kernels (64 registers;
-// their tiles need about 27 KB, and the extra warps hide more of the tile
-// pipeline's latency: 11 % faster on the limited Mach-3 step); in FP64 12
-// (P2: 168 registers, about 100 B of spills per thread, 17 % faster than
-// 8 warps at 236 registers on large meshes) and 16 (P1: 128 registers);
-// whatever the tile size.  LAT (FP64 only): 8 and 12 warps without spills,
-// for launches whose tiles all fit on the device at once, where a tile's
-// latency rather than the throughput of many sets the time.
-template <typename Real, int ORD, int BT, int LAT = 0>
+// Resident CTAs per SM the register allocation is held to: 24 warps per SM
+// for kernels with P2 tiles (80 registers; 128-element tiles at most 37 KB of
+// shared memory per CTA) and 32 for P1-only kernels (64 registers; their
+// tiles need about 27 KB, and the extra warps hide more of the tile
+// pipeline's latency: 11 % faster on the limited Mach-3 step), whatever the
+// tile size.
+template <int ORD, int BT>
 struct TiledOccupancy {
-    static constexpr int warps = sizeof(Real) == 8 ? (LAT ? (ORD == 1 ? 12 : 8) : (ORD == 1 ? 16 : 12))
-                                                   : (ORD == 1 ? 32 : 24);
+    static constexpr int warps = ORD == 1 ? 32 : 24;
     static constexpr int value = warps * 32 / BT > 0 ? warps * 32 / BT : 1;
 };
 
@@ -252,57 +256,30 @@ __device__ __forceinline__ void stage_prefetch(const StageArgs& a, const TileArg
     }
 }
 
-// A halo neighbour's trace (slot g < NG) or cell mean (slot NG) in the
-// staging area, over that neighbour's own staged state rows (entry h of the
-// [rows][HM] gather): FP32 one 16-byte row per slot (row g), FP64 two (rows
-// 2g and 2g + 1).  Each halo thread writes only its own entry, after it has
-// read the rows there.
-template <typename Real>
-__device__ __forceinline__ void put_htr(unsigned char* stg, int HM, int g, int h, const Real t[4]) {
-    if constexpr (sizeof(Real) == 8) {
-        double2* p = reinterpret_cast<double2*>(stg);
-        p[(2 * g) * HM + h] = make_double2(t[0], t[1]);
-        p[(2 * g + 1) * HM + h] = make_double2(t[2], t[3]);
-    } else {
-        reinterpret_cast<float4*>(stg)[g * HM + h] = make_float4(t[0], t[1], t[2], t[3]);
-    }
-}
-template <typename Real>
-__device__ __forceinline__ void get_htr(const unsigned char* stg, int HM, int g, int h, Real t[4]) {
-    if constexpr (sizeof(Real) == 8) {
-        const double2* p = reinterpret_cast<const double2*>(stg);
-        const double2 a = p[(2 * g) * HM + h], b = p[(2 * g + 1) * HM + h];
-        t[0] = a.x, t[1] = a.y, t[2] = b.x, t[3] = b.y;
-    } else {
-        const float4 a = reinterpret_cast<const float4*>(stg)[g * HM + h];
-        t[0] = a.x, t[1] = a.y, t[2] = a.z, t[3] = a.w;
+// Element x's state from the staging rows.
+template <int NB, int BT>
+__device__ __forceinline__ void load_staged(const unsigned char* stg, int x, float u[NB][4]) {
+    const float4* p = reinterpret_cast<const float4*>(stg);
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+        const float4 a = p[i * BT + x];
+        u[i][0] = a.x;
+        u[i][1] = a.y;
+        u[i][2] = a.z;
+        u[i][3] = a.w;
     }
 }
 
-// Element x's state from the staging rows.
-template <typename Real, int NB, int BT>
-__device__ __forceinline__ void load_staged(const unsigned char* stg, int x, Real u[NB][4]) {
-    if constexpr (sizeof(Real) == 8) {
-        const double2* p = reinterpret_cast<const double2*>(stg);
-#pragma unroll
-        for (int i = 0; i < NB; ++i) {
-            const double2 a = p[(2 * i) * BT + x], b = p[(2 * i + 1) * BT + x];
-            u[i][0] = a.x;
-            u[i][1] = a.y;
-            u[i][2] = b.x;
-            u[i][3] = b.y;
-        }
-    } else {
-        const float4* p = reinterpret_cast<const float4*>(stg);
-#pragma unroll
-        for (int i = 0; i < NB; ++i) {
-            const float4 a = p[i * BT + x];
-            u[i][0] = a.x;
-            u[i][1] = a.y;
-            u[i][2] = a.z;
-            u[i][3] = a.w;
-        }
-    }
+// One CTA per tile (no next tile of its own): the last warp prefetches the
+// tile a full device of CTAs further on, which a CTA yet to start will run,
+// so that its loads find L2 instead of HBM (980,000 triangles, FP32C P2:
+// 0.296 -> 0.289 ms per step; the FP64 kernel loses 2 % by it, its tiles
+// being longer than HBM's latency matters).
+template <typename Real, int BT>
+__device__ __forceinline__ void prefetch_ahead(const StageArgs& a, const TileArgs& ta, int nxt, int ntiles) {
+    if (threadIdx.x != BT - 32 || nxt < ntiles) return;
+    const int t = (int)blockIdx.x + ta.ahead;
+    if (ta.ahead > 0 && t < ntiles) stage_prefetch<Real, true>(a, ta, __ldg(ta.desc + 2 * t), __ldg(ta.desc + 2 * t + 1));
 }
 
 // The part of a tile's work that needs only its descriptors, J^-1 rows and
@@ -323,16 +300,7 @@ __device__ __forceinline__ TilePre<Real> tile_pre(const StageArgs& a, const Tile
     constexpr int NC = TiledLayout<Real, BT>::NC;
     const int tid = threadIdx.x;
     TilePre<Real> t;
-    // far-field / reference state by value (a pointer into the parameter
-    // block would put the parameter array in local memory)
-    double fs[4];
-    if (a.far_sid) {
-        const double* p = a.far_sid + 4 * d0.z;
-        fs[0] = p[0], fs[1] = p[1], fs[2] = p[2], fs[3] = p[3];
-    } else {
-        fs[0] = a.far[0], fs[1] = a.far[1], fs[2] = a.far[2], fs[3] = a.far[3];
-    }
-    t.rs = ref_state<Real>(fs, a.gamma);
+    t.rs = ref_state(a.ref32, d0.z);
     // the halo and task lists (L2 hits: prefetched with the tile's rows)
     const int h0 = d1.x, nh = d1.y, t0 = d1.z, nt = d1.w;
     int4* s_code = reinterpret_cast<int4*>(smem_raw + TiledLayout<Real, BT>::code_off);  // [BT]
@@ -369,13 +337,26 @@ __device__ __forceinline__ TilePre<Real> tile_pre(const StageArgs& a, const Tile
     return t;
 }
 
+// The neighbour-side edge tables (runtime edge index) of the orders a kernel
+// runs, from global memory into shared memory: [0] the P2 (or only) order's,
+// [1] P1's in a mixed kernel.
+template <int ORD, int NQ2, int BT, typename T>
+__device__ __forceinline__ void load_edge_table(const T (*g)[3 * kMaxNG * kMaxNB], T (*s)[3 * kMaxNG * kMaxNB]) {
+    constexpr int P1 = cfg_index(3, 2);
+    constexpr int n = ORD == 1 ? 3 * 2 * 3 : 3 * 3 * 6;
+    for (int x = threadIdx.x; x < n; x += BT) s[0][x] = __ldg(&g[ORD == 1 ? P1 : cfg_index(NQ2, 3)][x]);
+    if constexpr (ORD == 3)
+        for (int x = threadIdx.x; x < 3 * 2 * 3; x += BT) s[1][x] = __ldg(&g[P1][x]);
+}
+
 // Returns, when the stage is followed by the TVB limiter (a.tile_flags set),
 // whether the limiter may change this thread's element (tvb_keeps fails).
 template <typename Real, int NB, int NQ, int NG, int FLUX, int MODE, int BT>
 __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& ta, const int4 d0,
                                            const int4 d1, unsigned char* smem_raw, unsigned char* stg,
                                            const int nxt, const int ntiles, uint64_t* bar,
-                                           const TilePre<Real>& pre, Real (*s_red)[3], const double* s_dt) {
+                                           const TilePre<Real>& pre, const float2* s_ephi, Real (*s_red)[3],
+                                           const double* s_dt) {
     constexpr int CFG = cfg_index(NQ, NG);
     using V4 = Vec4<Real>;
     const Tab<Real>& tb = tab<Real>(CFG);
@@ -388,19 +369,12 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
     constexpr int MEANS = FLUX == RKDG_FLUX_LLF ? 1 : 0;                   // LLF needs cell means
     V4* s_mean = s_tr + 3 * NG * BT;                                       // [BT] (LLF)
     // halo traces and means: in the staging rows, over each neighbour's own
-    // staged state (put_htr / get_htr; FP32 also through these pointers,
-    // trace g of halo h in row g, entry h)
+    // staged state (trace g of halo h in row g, entry h; its mean in row NG).
+    // Each halo thread writes only its own entry, after it has read the rows
+    // there.
     V4* s_htr = reinterpret_cast<V4*>(stg);
     V4* s_hmean = s_htr + NG * HM;
-    constexpr bool PK = sizeof(Real) == 4;  // FP32: lane-pair arithmetic, paired tables
-    const Tab2& t2 = c_tab_f2[CFG];
-    using SE = typename std::conditional<PK, float2, Real>::type;
-    __shared__ SE s_ephi[3][NG][NB];  // neighbour-side edge table (runtime edge index)
-    for (int x = threadIdx.x; x < 3 * NG * NB; x += BT) {
-        int k = x / (NG * NB), g = (x / NB) % NG, i = x % NB;
-        if constexpr (PK) s_ephi[k][g][i] = t2.ephi[k][g][i];
-        else s_ephi[k][g][i] = tb.ephi[k][g][i];
-    }
+    const Tab2& t2 = c_tab_f2[CFG];   // paired tables of the lane-pair arithmetic
     const int sid = d0.z;
     StepCtl* ctl = a.ctl + sid;
 
@@ -412,16 +386,13 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
     const int sx = active ? tid : 0;  // staging row index
     const Real* __restrict__ U = static_cast<const Real*>(a.U);
     const Real gamma = (Real)a.gamma, gm1 = gamma - Real(1);
-    // FP32: traces and fluxes in deviation form about the reference state
-    constexpr bool DEV = stores_deviation<Real>();
+    // traces and fluxes in deviation form about the reference state; a
+    // stored mean is the deviation from it
     const RefState<Real> rs = pre.rs;
     const Real far[4] = {rs.rho, rs.mx, rs.my, rs.E};
-    Real refv[4];  // the offset of a stored mean (FP32: the far field)
-#pragma unroll
-    for (int v = 0; v < 4; ++v) refv[v] = DEV ? far[v] : Real(0);
 
     // ------------------------------------------------------------ phase A
-    constexpr int SR = NB * (int)(sizeof(Real) / 4);  // 16-byte rows of a state
+    constexpr int SR = NB;  // 16-byte rows of a state
     const int nh = d1.y, nt = d1.w;
     const int2* hh = pre.hh;
     Real R[NB][4];
@@ -429,11 +400,8 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
     const double det = pre.det;
     const Real inv_area = pre.inv_area;
     const Real j00 = pre.j00, j01 = pre.j01, j10 = pre.j10, j11 = pre.j11;  // rows of 2 area J^-1
-    // psi_0 is the constant K00 at every volume and edge point: its term is
-    // formed once per state
-    const Real k00 = tb.vphi[0][0];
     {
-        load_staged<Real, NB, BT>(stg, sx, u);
+        load_staged<NB, BT>(stg, sx, u);
         __syncthreads();  // staged rows consumed: the area takes the halo states
         {
             const char* Ub = static_cast<const char*>(a.U);
@@ -450,89 +418,35 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
         {
             Real mfull[4];
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                mfull[v] = u[0][v] + refv[v];  // the cell mean itself
-                if constexpr (!DEV) u[0][v] = mfull[v];
-            }
+            for (int v = 0; v < 4; ++v) mfull[v] = u[0][v] + far[v];  // the cell mean itself
             if constexpr (MEANS) put4(s_mean + tid, mfull);
         }
 #pragma unroll
         for (int i = 0; i < NB; ++i)
 #pragma unroll
             for (int v = 0; v < 4; ++v) R[i][v] = Real(0);
-        Real c0[4];
-        if constexpr (PK) {
-            const float2 kk = make_float2(k00, k00);
-            set4(c0, f2mul(kk, lo2(u[0])), f2mul(kk, hi2(u[0])));
-        } else {
-#pragma unroll
-            for (int v = 0; v < 4; ++v) c0[v] = k00 * u[0][v];
-        }
-        // FP32: the quadrature loop is unrolled by two only (a smaller body
-        // keeps the instruction cache warm across the CTAs on an SM; full
-        // unrolling is 2 % slower, none 1 %); FP64 unrolls it.  Each product
-        // is its own fused multiply-add, and psi_1 (a function of xi alone)
-        // has no eta-derivative term.
-        constexpr int VOL_UNROLL = sizeof(Real) == 4 ? 2 : NQ;
-#pragma unroll VOL_UNROLL
+        // the quadrature loop is unrolled by two only (a smaller body keeps
+        // the instruction cache warm across the CTAs on an SM; full unrolling
+        // is 2 % slower, none 1 %).  psi_0 is one at every point and psi_1 (a
+        // function of xi alone) has no eta-derivative term.
+#pragma unroll 2
         for (int q = 0; q < NQ; ++q) {
             Real w[4];
-            if constexpr (PK) {
-                comb_rows<NB>(t2.vphi[q], u, lo2(c0), hi2(c0), w);
-            } else {
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    Real s = c0[v];
-#pragma unroll
-                    for (int i = 1; i < NB; ++i) s += tb.vphi[q][i] * u[i][v];
-                    w[v] = s;
-                }
-            }
+            comb_rows<NB>(t2.vphi[q], u, lo2(u[0]), hi2(u[0]), w);
             Real fx[4], fy[4];
-            if constexpr (DEV) {
-                // flux deviations through the rows of 2 area J^-1
-                const DevPrims<Real> pw = dev_prims(w, rs, gm1);
-                dev_flux(w, pw, rs, j00, j01, fx);
-                dev_flux(w, pw, rs, j10, j11, fy);
-            } else {
-                // the fluxes through the rows of 2 area J^-1, by their
-                // contravariant speeds
-                const Real ri = rcp_(w[0]);
-                const Real vx = w[1] * ri, vy = w[2] * ri;
-                const Real p = gm1 * (w[3] - Real(0.5) * (w[1] * vx + w[2] * vy));
-                const Real q0 = j00 * vx + j01 * vy, q1 = j10 * vx + j11 * vy, h = w[3] + p;
-                fx[0] = w[0] * q0, fx[1] = w[1] * q0 + j00 * p, fx[2] = w[2] * q0 + j01 * p, fx[3] = h * q0;
-                fy[0] = w[0] * q1, fy[1] = w[1] * q1 + j10 * p, fy[2] = w[2] * q1 + j11 * p, fy[3] = h * q1;
-            }
-            if constexpr (PK) {
-                acc_rows<1, NB>(R, fx, t2.vdxi[q]);
-                acc_rows<2, NB>(R, fy, t2.veta[q]);
-            } else {
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-#pragma unroll
-                    for (int i = 1; i < NB; ++i) R[i][v] += fx[v] * tb.vdxi[q][i];
-#pragma unroll
-                    for (int i = 2; i < NB; ++i) R[i][v] += fy[v] * tb.veta[q][i];
-                }
-            }
+            // flux deviations through the rows of 2 area J^-1
+            const DevPrims<Real> pw = dev_prims(w, rs, gm1);
+            dev_flux(w, pw, rs, j00, j01, fx);
+            dev_flux(w, pw, rs, j10, j11, fy);
+            acc_rows<1, NB>(R, fx, t2.vdxi[q]);
+            acc_rows<2, NB>(R, fy, t2.veta[q]);
         }
 #pragma unroll
         for (int k = 0; k < 3; ++k)
 #pragma unroll
             for (int g = 0; g < NG; ++g) {
                 Real t[4];
-                if constexpr (PK) {
-                    comb_rows<NB>(t2.ephi[k][g], u, lo2(c0), hi2(c0), t);
-                } else {
-#pragma unroll
-                    for (int v = 0; v < 4; ++v) {
-                        Real s = c0[v];
-#pragma unroll
-                        for (int i = 1; i < NB; ++i) s += tb.ephi[k][g][i] * u[i][v];
-                        t[v] = s;
-                    }
-                }
+                comb_rows<NB>(t2.ephi[k][g], u, lo2(u[0]), hi2(u[0]), t);
                 put4(s_tr + (k * NG + g) * BT + tid, t);
             }
     }
@@ -544,54 +458,24 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
             const int h = tid + r * BT;
             if (h < nh) {
                 Real un[NB][4];
-                if constexpr (sizeof(Real) == 8) {
-                    const double2* p = reinterpret_cast<const double2*>(stg);
+                const float4* p = reinterpret_cast<const float4*>(stg);
 #pragma unroll
-                    for (int i = 0; i < NB; ++i) {
-                        const double2 x = p[(2 * i) * HM + h], y = p[(2 * i + 1) * HM + h];
-                        un[i][0] = x.x, un[i][1] = x.y, un[i][2] = y.x, un[i][3] = y.y;
-                    }
-                } else {
-                    const float4* p = reinterpret_cast<const float4*>(stg);
-#pragma unroll
-                    for (int i = 0; i < NB; ++i) {
-                        const float4 x = p[i * HM + h];
-                        un[i][0] = x.x, un[i][1] = x.y, un[i][2] = x.z, un[i][3] = x.w;
-                    }
+                for (int i = 0; i < NB; ++i) {
+                    const float4 x = p[i * HM + h];
+                    un[i][0] = x.x, un[i][1] = x.y, un[i][2] = x.z, un[i][3] = x.w;
                 }
-                {
+                if constexpr (MEANS) {
                     Real mfull[4];
 #pragma unroll
-                    for (int v = 0; v < 4; ++v) {
-                        mfull[v] = un[0][v] + refv[v];
-                        if constexpr (!DEV) un[0][v] = mfull[v];
-                    }
-                    if constexpr (MEANS) put_htr<Real>(stg, HM, NG, h, mfull);
+                    for (int v = 0; v < 4; ++v) mfull[v] = un[0][v] + far[v];
+                    put4(s_hmean + h, mfull);
                 }
                 const int he = hh[r].y;
-                Real c0[4];
-                if constexpr (PK) {
-                    const float2 kk = make_float2(k00, k00);
-                    set4(c0, f2mul(kk, lo2(un[0])), f2mul(kk, hi2(un[0])));
-                } else {
-#pragma unroll
-                    for (int v = 0; v < 4; ++v) c0[v] = k00 * un[0][v];
-                }
 #pragma unroll
                 for (int g = 0; g < NG; ++g) {
                     Real t[4];
-                    if constexpr (PK) {
-                        comb_rows<NB>(s_ephi[he][g], un, lo2(c0), hi2(c0), t);
-                    } else {
-#pragma unroll
-                        for (int v = 0; v < 4; ++v) {
-                            Real s = c0[v];
-#pragma unroll
-                            for (int i = 1; i < NB; ++i) s += s_ephi[he][g][i] * un[i][v];
-                            t[v] = s;
-                        }
-                    }
-                    put_htr<Real>(stg, HM, g, h, t);
+                    comb_rows<NB>(s_ephi + (he * NG + g) * NB, un, lo2(un[0]), hi2(un[0]), t);
+                    put4(s_htr + g * HM + h, t);
                 }
             }
         }
@@ -602,6 +486,7 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
         nd0 = __ldg(ta.desc + 2 * nxt);
         stage_prefetch<Real, true>(a, ta, nd0, __ldg(ta.desc + 2 * nxt + 1));
     }
+    prefetch_ahead<Real, BT>(a, ta, nxt, ntiles);
 
     // ------------------------------------------------------------ phase B
     {
@@ -619,9 +504,7 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
             if constexpr (MEANS) {
                 get4(s_mean + le, mL);
                 if (kind == EDGE_BOUNDARY) ghost<Real>(se, mL, far, nx, ny, mR);
-                else if constexpr (sizeof(Real) == 4) get4(kind == EDGE_HALO ? s_hmean + idx : s_mean + idx, mR);
-                else if (kind == EDGE_HALO) get_htr<Real>(stg, HM, NG, idx, mR);
-                else get4(s_mean + idx, mR);
+                else get4(kind == EDGE_HALO ? s_hmean + idx : s_mean + idx, mR);
             }
             Real alpha = Real(0);
             if constexpr (FLUX == RKDG_FLUX_LLF) {
@@ -642,55 +525,26 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
                 get4(slot, uL);
                 // the neighbour's point NG-1-g on its edge se pairs with ours
                 // (src/kernelfunctions.cu:545-549)
-                V4* nslot = sizeof(Real) == 4 && kind == EDGE_HALO ? s_htr + (NG - 1 - g) * HM + idx
-                                                                   : s_tr + (se * NG + NG - 1 - g) * BT + idx;
-                if (kind == EDGE_BOUNDARY) {
-                    if constexpr (DEV) ghost_dev<Real>(se, uL, rs, nx, ny, uR);
-                    else ghost<Real>(se, uL, far, nx, ny, uR);
-                }
-                else if (sizeof(Real) == 8 && kind == EDGE_HALO) get_htr<Real>(stg, HM, NG - 1 - g, idx, uR);
+                V4* nslot = kind == EDGE_HALO ? s_htr + (NG - 1 - g) * HM + idx : s_tr + (se * NG + NG - 1 - g) * BT + idx;
+                if (kind == EDGE_BOUNDARY) ghost_dev<Real>(se, uL, rs, nx, ny, uR);
                 else get4(nslot, uR);
                 Real fh[4], fn[4];  // the flux out of this side and into the neighbour
                 if (FLUX == RKDG_FLUX_LLF) {
                     Real fL[4], fR[4];
-                    if constexpr (DEV) {
-                        dev_flux(uL, dev_prims(uL, rs, gm1), rs, Nx, Ny, fL);
-                        dev_flux(uR, dev_prims(uR, rs, gm1), rs, Nx, Ny, fR);
-                    } else {
-                        Real pL, pR;
-                        normal_flux<Real>(uL, Nx, Ny, gm1, fL, pL);
-                        normal_flux<Real>(uR, Nx, Ny, gm1, fR, pR);
-                    }
-                    if constexpr (PK) {
-                        const float2 na = make_float2(-alpha, -alpha);
-                        const float2 tl = f2fma(na, f2sub(lo2(uR), lo2(uL)), f2add(lo2(fL), lo2(fR)));
-                        const float2 th = f2fma(na, f2sub(hi2(uR), hi2(uL)), f2add(hi2(fL), hi2(fR)));
-                        const float2 hp = make_float2(0.5f, 0.5f), hn = make_float2(-0.5f, -0.5f);
-                        set4(fh, f2mul(hp, tl), f2mul(hp, th));
-                        set4(fn, f2mul(hn, tl), f2mul(hn, th));
-                    } else {
-#pragma unroll
-                        for (int v = 0; v < 4; ++v) {
-                            const Real t = fL[v] + fR[v] - alpha * (uR[v] - uL[v]);
-                            fh[v] = Real(0.5) * t;
-                            fn[v] = Real(-0.5) * t;
-                        }
-                    }
+                    dev_flux(uL, dev_prims(uL, rs, gm1), rs, Nx, Ny, fL);
+                    dev_flux(uR, dev_prims(uR, rs, gm1), rs, Nx, Ny, fR);
+                    const float2 na = make_float2(-alpha, -alpha);
+                    const float2 tl = f2fma(na, f2sub(lo2(uR), lo2(uL)), f2add(lo2(fL), lo2(fR)));
+                    const float2 th = f2fma(na, f2sub(hi2(uR), hi2(uL)), f2add(hi2(fL), hi2(fR)));
+                    const float2 hp = make_float2(0.5f, 0.5f), hn = make_float2(-0.5f, -0.5f);
+                    set4(fh, f2mul(hp, tl), f2mul(hp, th));
+                    set4(fn, f2mul(hn, tl), f2mul(hn, th));
                 } else {
                     Real f[4];
-                    if constexpr (DEV) hllc_dev<Real>(uL, uR, nx, ny, gamma, rs, f);
-                    else hllc<Real>(uL, uR, nx, ny, gamma, f);
-                    if constexpr (PK) {
-                        const float2 l = make_float2(len, len), nl = make_float2(-len, -len);
-                        set4(fh, f2mul(lo2(f), l), f2mul(hi2(f), l));
-                        set4(fn, f2mul(lo2(f), nl), f2mul(hi2(f), nl));
-                    } else {
-#pragma unroll
-                        for (int v = 0; v < 4; ++v) {
-                            fh[v] = f[v] * len;
-                            fn[v] = f[v] * -len;
-                        }
-                    }
+                    hllc_dev<Real>(uL, uR, nx, ny, gamma, rs, f);
+                    const float2 l = make_float2(len, len), nl = make_float2(-len, -len);
+                    set4(fh, f2mul(lo2(f), l), f2mul(hi2(f), l));
+                    set4(fn, f2mul(lo2(f), nl), f2mul(hi2(f), nl));
                 }
                 // each slot of an edge is read by this task alone: the
                 // computing side's slot takes the flux, an in-tile
@@ -714,14 +568,7 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
         for (int g = 0; g < NG; ++g) {
             Real f[4];
             get4(s_tr + (k * NG + g) * BT + tid, f);
-            if constexpr (PK) {
-                acc_rows<0, NB>(R, f, t2.nephiw[k][g]);
-            } else {
-#pragma unroll
-                for (int v = 0; v < 4; ++v)
-#pragma unroll
-                    for (int i = 0; i < NB; ++i) R[i][v] -= f[v] * tb.ephiw[k][g][i];
-            }
+            acc_rows<0, NB>(R, f, t2.nephiw[k][g]);
         }
 
     Real* __restrict__ Uout = static_cast<Real*>(a.Unew);
@@ -741,42 +588,28 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
     const Real dt = (Real)(dtd * det), cb = (Real)a.b;
     Real u0m[4] = {Real(0), Real(0), Real(0), Real(0)};
     // RKDG_FP32C (comp): row 0 is updated in FP64 below, not here
-    constexpr bool comp = PK && (MODE & MODE_STAGE_COMP);
+    constexpr bool comp = (MODE & MODE_STAGE_COMP) != 0;
     {
         load_state<Real, NB>(U, a.ld, ee, u);  // stored values (L2 hit)
         if (a.U0 != nullptr) {
             Real u0[NB][4];
             load_state<Real, NB>(static_cast<const Real*>(a.U0), a.ld, ee, u0);
-            if constexpr (PK) {
-                const float2 dt2 = make_float2(dt, dt), cb2 = make_float2(cb, cb);
+            const float2 dt2 = make_float2(dt, dt), cb2 = make_float2(cb, cb);
 #pragma unroll
-                for (int i = 0; i < NB; ++i) {
-                    const float2 l = f2fma(cb2, f2fma(dt2, lo2(R[i]), f2sub(lo2(u[i]), lo2(u0[i]))), lo2(u0[i]));
-                    const float2 h = f2fma(cb2, f2fma(dt2, hi2(R[i]), f2sub(hi2(u[i]), hi2(u0[i]))), hi2(u0[i]));
-                    if (i > 0 || !comp) set4(R[i], l, h);
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < NB; ++i)
-#pragma unroll
-                    for (int v = 0; v < 4; ++v) R[i][v] = u0[i][v] + cb * ((u[i][v] - u0[i][v]) + dt * R[i][v]);
+            for (int i = 0; i < NB; ++i) {
+                const float2 l = f2fma(cb2, f2fma(dt2, lo2(R[i]), f2sub(lo2(u[i]), lo2(u0[i]))), lo2(u0[i]));
+                const float2 h = f2fma(cb2, f2fma(dt2, hi2(R[i]), f2sub(hi2(u[i]), hi2(u0[i]))), hi2(u0[i]));
+                if (i > 0 || !comp) set4(R[i], l, h);
             }
 #pragma unroll
             for (int v = 0; v < 4; ++v) u0m[v] = u0[0][v];
         } else {
-            if constexpr (PK) {
-                const float2 dt2 = make_float2(dt, dt), cb2 = make_float2(cb, cb);
+            const float2 dt2 = make_float2(dt, dt), cb2 = make_float2(cb, cb);
 #pragma unroll
-                for (int i = 0; i < NB; ++i) {
-                    const float2 l = f2mul(cb2, f2fma(dt2, lo2(R[i]), lo2(u[i])));
-                    const float2 h = f2mul(cb2, f2fma(dt2, hi2(R[i]), hi2(u[i])));
-                    if (i > 0 || !comp) set4(R[i], l, h);
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < NB; ++i)
-#pragma unroll
-                    for (int v = 0; v < 4; ++v) R[i][v] = cb * (u[i][v] + dt * R[i][v]);
+            for (int i = 0; i < NB; ++i) {
+                const float2 l = f2mul(cb2, f2fma(dt2, lo2(R[i]), lo2(u[i])));
+                const float2 h = f2mul(cb2, f2fma(dt2, hi2(R[i]), hi2(u[i])));
+                if (i > 0 || !comp) set4(R[i], l, h);
             }
         }
     }
@@ -827,7 +660,7 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
             bool bad;
             Real m[4], len[3];
 #pragma unroll
-            for (int v = 0; v < 4; ++v) m[v] = R[0][v] + refv[v];
+            for (int v = 0; v < 4; ++v) m[v] = R[0][v] + far[v];
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 const Real Nx = s_nrm[(NC * k + 0) * BT + tid], Ny = s_nrm[(NC * k + 1) * BT + tid];
@@ -859,7 +692,7 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
         // J^-1: the columns of J are (j11, -j10) and (-j01, j00))
         Real mean[4], tmax = Real(0);
 #pragma unroll
-        for (int v = 0; v < 4; ++v) mean[v] = R[0][v] + refv[v];
+        for (int v = 0; v < 4; ++v) mean[v] = R[0][v] + far[v];
 #pragma unroll
         for (int k = 0; k < 3; ++k)
 #pragma unroll
@@ -875,11 +708,11 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
 // The tile's maxima from s_red into its solve's control block (one thread,
 // after the barrier that closes the tile; bits of a non-negative double
 // order like the values).
-template <typename Real, int BT>
+template <typename Real, int NT>
 __device__ __forceinline__ void tile_maxima_atomic(const StageArgs& a, StepCtl* ctl, const Real (*s_red)[3]) {
     Real w = s_red[0][0], m0 = s_red[0][1], m1 = s_red[0][2];
 #pragma unroll
-    for (int k = 1; k < BT / 32; ++k) {
+    for (int k = 1; k < NT / 32; ++k) {
         w = fmax(w, s_red[k][0]);
         m0 = fmax(m0, s_red[k][1]);
         m1 = fmax(m1, s_red[k][2]);
@@ -896,9 +729,10 @@ __device__ __forceinline__ void tile_maxima_atomic(const StageArgs& a, StepCtl* 
 // BT: elements per tile = threads per CTA.
 // A barrier wait that times out sets bit 1 of the solve's error word and
 // ends the CTA (all threads together).
-template <typename Real, int NQ2, int FLUX, int MODE, int ORD, int BT, int LAT = 0>
-__global__ void __launch_bounds__(BT, TiledOccupancy<Real, ORD, BT, LAT>::value)
+template <int NQ2, int FLUX, int MODE, int ORD, int BT>
+__global__ void __launch_bounds__(BT, TiledOccupancy<ORD, BT>::value)
     tiled_stage_kernel(const StageArgs a, const TileArgs ta) {
+    using Real = float;
     using SM = TiledSmem<Real, ORD, FLUX, BT>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t s_bar;
@@ -908,19 +742,17 @@ __global__ void __launch_bounds__(BT, TiledOccupancy<Real, ORD, BT, LAT>::value)
     const int ntiles = ta.ntiles_dev ? *ta.ntiles_dev : ta.ntiles;
     int tile = blockIdx.x;
     if (tile >= ntiles) return;
+    // every thread's descriptor load is in flight while the barrier is set
+    // up; nobody waits for the thread that issues the copies
+    int4 d0 = __ldg(ta.desc + 2 * tile), d1 = __ldg(ta.desc + 2 * tile + 1);
     if (threadIdx.x == 0) mbar_init(&s_bar, 1);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        const int4 fd = __ldg(ta.desc + 2 * tile);
-        stage_copy<Real, BT>(a, fd, stg, &s_bar);
-        // the first tile's table prefetch: a gain for FP64 (measured at two
-        // CTAs per SM), a loss for FP32
-        if constexpr (sizeof(Real) == 8) stage_prefetch<Real, false>(a, ta, fd, __ldg(ta.desc + 2 * tile + 1));
-    }
+    if (threadIdx.x == 0) stage_copy<Real, BT>(a, d0, stg, &s_bar);
+    __shared__ float2 s_ephi[ORD == 3 ? 2 : 1][3 * kMaxNG * kMaxNB];
+    load_edge_table<ORD, NQ2, BT>(g_ephi_f2, s_ephi);  // (read after later barriers)
     const double2* jinv2 = reinterpret_cast<const double2*>(a.jinv);
     uint32_t parity = 0;
-    for (; tile < ntiles; tile += gridDim.x) {
-        const int4 d0 = __ldg(ta.desc + 2 * tile), d1 = __ldg(ta.desc + 2 * tile + 1);
+    for (;; tile += gridDim.x, d0 = __ldg(ta.desc + 2 * tile), d1 = __ldg(ta.desc + 2 * tile + 1)) {
         const int nxt = tile + gridDim.x;
         // this thread's J^-1 rows and edge codes, and the work that needs
         // only them, while the state rows arrive
@@ -937,16 +769,17 @@ __global__ void __launch_bounds__(BT, TiledOccupancy<Real, ORD, BT, LAT>::value)
         }
         parity ^= 1u;
         if (done) {  // finished solve: pass the tile on
-            if (threadIdx.x == 0 && nxt < ntiles) stage_copy<Real, BT>(a, __ldg(ta.desc + 2 * nxt), stg, &s_bar);
+            if (nxt >= ntiles) return;
+            if (threadIdx.x == 0) stage_copy<Real, BT>(a, __ldg(ta.desc + 2 * nxt), stg, &s_bar);
             continue;
         }
         bool need;
         if (ORD == 2 || (ORD == 3 && d0.w == 2))
             need = tile_stage<Real, 6, NQ2, 3, FLUX, MODE, BT>(a, ta, d0, d1, smem_raw, stg, nxt, ntiles, &s_bar, pre,
-                                                              s_red, &s_dt);
+                                                              s_ephi[0], s_red, &s_dt);
         else
             need = tile_stage<Real, 3, 3, 2, FLUX, MODE, BT>(a, ta, d0, d1, smem_raw, stg, nxt, ntiles, &s_bar, pre,
-                                                            s_red, &s_dt);
+                                                            s_ephi[ORD == 3 ? 1 : 0], s_red, &s_dt);
         // shared memory is reused by the next tile (with the limiter the
         // barrier also ORs its test over the tile)
         if constexpr (MODE & MODE_LIMITED) {
@@ -960,5 +793,6 @@ __global__ void __launch_bounds__(BT, TiledOccupancy<Real, ORD, BT, LAT>::value)
         }
         if (MODE != MODE_RESIDUAL && a.last_stage && threadIdx.x == 0)
             tile_maxima_atomic<Real, BT>(a, a.ctl + d0.z, s_red);
+        if (nxt >= ntiles) return;
     }
 }
