@@ -50,6 +50,8 @@ struct rkdg_ctx {
     int pending_out = -1;
     std::unique_ptr<std::ofstream> reslog;  // residual history file (rkdg_set_residual_log)
     bool graph_monitor = false;  // the captured step forms the residual monitor
+    bool resident = false;       // whole steps run in the resident kernel
+    ResidentWork rw;             // its exchange buffers
 };
 
 namespace {
@@ -221,6 +223,16 @@ void enqueue_step(rkdg_ctx* c, bool monitor) {
     }
 }
 
+// `steps` whole steps (at most kResidentSteps) in one launch, with the state
+// in buffer 0
+void enqueue_resident(rkdg_ctx* c, int steps, bool monitor) {
+    StageArgs a = base_args(c);
+    a.Unew = c->d.U[0];
+    a.far_sid = c->d.far;
+    launch_resident(a, c->tiles, c->p.limiter == RKDG_LIMITER_TVB ? c->d.lim : nullptr, c->rw, c->p.order, c->p.nq,
+                    c->p.flux, kprec(c), c->p.rk, steps, monitor, c->stream);
+}
+
 constexpr int kGraphSteps = 8;
 
 // A graph of `steps` whole steps on the context's stream.
@@ -304,6 +316,7 @@ void destroy_ctx(rkdg_ctx* c) {
     cudaFree(c->d.ctl);
     cudaFree(c->d.far);
     cudaFree(c->d.ref32);
+    for (void* p : {c->rw.trace, c->rw.mean, (void*)c->rw.slot, (void*)c->rw.sums}) cudaFree(p);
     cudaFree(c->d.tcode);
     cudaFree(c->d.tdesc);
     cudaFree(c->d.halo);
@@ -464,6 +477,31 @@ int create_ctx(const rkdg_mesh_desc* mesh, const rkdg_params* params, int32_t n_
                 c->d.tile_list = (int*)dev_alloc(c, nl);
                 RKDG_CUDA_TRY(cudaMemsetAsync(c->d.tile_flags, 0, nf, c->stream));
                 RKDG_CUDA_TRY(cudaMemsetAsync(c->d.tile_list, 0, nl, c->stream));
+            }
+            const bool lim = params->limiter == RKDG_LIMITER_TVB, comp = params->precision == RKDG_FP32C;
+            std::vector<int32_t> slot;
+            if (n_owned < 0 && tt.ntiles <= resident_tiles(kprec(c), params->order, params->nq, params->flux, lim,
+                                                           comp, tt.max_halo)) {
+                c->resident = true;
+                (kprec(c) == RKDG_FP64 ? upload_resident_tables_fp64 : upload_resident_tables_fp32)(params->nq, params->ng);
+                slot.assign((size_t)3 * ld, -1);
+                for (size_t h = 0; h < tt.halo.size() / 2; ++h)
+                    slot[(size_t)tt.halo[2 * h + 1] * ld + tt.halo[2 * h]] = (int32_t)h;
+                ResidentWork& w = c->rw;
+                w.slots = std::max(1, (int)(tt.halo.size() / 2));
+                w.slot = (int*)dev_alloc(c, sizeof(int32_t) * slot.size());
+                RKDG_CUDA_TRY(cudaMemcpyAsync(w.slot, slot.data(), sizeof(int32_t) * slot.size(),
+                                              cudaMemcpyHostToDevice, c->stream));
+                // two parities, two halves per 16-byte row
+                const size_t row = (size_t)4 * 16 * w.slots * (kprec(c) == RKDG_FP64 ? 2 : 1);
+                const size_t nt = row * (params->ng + (params->flux == RKDG_FLUX_LLF ? 1 : 0));
+                w.trace = dev_alloc(c, nt);
+                RKDG_CUDA_TRY(cudaMemsetAsync(w.trace, 0, nt, c->stream));
+                if (lim) {
+                    w.mean = dev_alloc(c, row);
+                    RKDG_CUDA_TRY(cudaMemsetAsync(w.mean, 0, row, c->stream));
+                }
+                w.sums = (unsigned char*)dev_alloc(c, kResidentSums);
             }
             sync(c);  // host tables go out of scope
         }
@@ -812,7 +850,8 @@ int rkdg_step(rkdg_ctx* c, double dt, double* dt_used, double* monitor) {
         c->h_ctl->t_final = 0.0;
         c->h_ctl->done = 0;
         push_ctl(c);
-        enqueue_step(c, true);
+        if (c->resident) enqueue_resident(c, 1, true);
+        else enqueue_step(c, true);
         c->wave_valid = true;
         pull_ctl(c);
         check_error_flag(c);
@@ -840,6 +879,30 @@ int rkdg_advance(rkdg_ctx* c, int32_t nsteps, double t_final, double* t, int32_t
         c->h_ctl->t_final = t_final > 0 ? t_final : 0.0;
         c->h_ctl->done = 0;
         push_ctl(c);
+        if (c->resident) {
+            int left = nsteps;
+            while (left > 0) {
+                const int n = c->reslog ? 1 : std::min(left, kResidentSteps);
+                const int before = c->h_ctl->step;
+                enqueue_resident(c, n, (bool)c->reslog);
+                left -= n;
+                // with a final time, stop once the device says done; the
+                // history needs every step's monitor
+                if (c->reslog || (t_final > 0 && left > 0)) {
+                    pull_ctl(c);
+                    if (c->reslog && (c->h_ctl->step == before || c->h_ctl->error)) break;  // done or failed
+                    log_residual(c);
+                    if (!c->reslog && (c->h_ctl->done || c->h_ctl->error)) break;
+                }
+            }
+            if (c->reslog) c->reslog->flush();
+            c->wave_valid = true;
+            pull_ctl(c);
+            check_error_flag(c);
+            if (t) *t = c->h_ctl->t;
+            if (steps_done) *steps_done = c->h_ctl->step - step0;
+            return;
+        }
         if (c->graph && c->graph_monitor != (bool)c->reslog) {  // the history needs the monitor
             cudaGraphExecDestroy(c->graph);
             c->graph = nullptr;

@@ -249,6 +249,31 @@ inline int state_rows(int precision, int nb) {
 // arithmetic type of a kernel (RKDG_FP64 or RKDG_FP32; kernel_prec maps the
 // RKDG_FP32C setting to RKDG_FP32).
 void upload_tables(int nq, int ng);
+// Whole steps of one solve in one cooperative launch (resident.cuh), for
+// solves of at most resident_tiles(...) tiles (0: none; the tile list's halo
+// lists must fit a CTA) in the locality order, element 0 first.
+struct ResidentWork {            // a context's exchange buffers
+    int* slot = nullptr;         // [3][ld] the halo entry (in any tile's list) that reads each element edge, or -1
+    int slots = 0;               // halo entries
+    void* trace = nullptr;       // [2][rows][2][slots] 16 bytes, zero before the first launch
+    void* mean = nullptr;        // with the limiter, likewise
+    unsigned char* sums = nullptr;  // per-step maxima and counts of one launch, the monitor
+    unsigned epoch = 0;          // stages numbered so far
+};
+constexpr int kResidentSteps = 64;  // most steps of one launch
+constexpr size_t kResidentSums = kResidentSteps * 12 + 16;
+int resident_tiles(int prec, int order, int nq, int flux, bool limiter, bool comp, int max_halo);
+// its tables (each CUDA translation unit holds its own)
+void upload_resident_tables_fp32(int nq, int ng);
+void upload_resident_tables_fp64(int nq, int ng);
+void launch_resident(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
+                     int flux, int prec, int rk, int steps, bool monitor, cudaStream_t stream);
+int resident_tiles_fp32(int order, int nq, int flux, bool limiter, bool comp, int max_halo);
+int resident_tiles_fp64(int order, int nq, int flux, bool limiter, bool comp, int max_halo);
+void launch_resident_fp32(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
+                          int flux, int rk, int steps, bool monitor, cudaStream_t stream);
+void launch_resident_fp64(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
+                          int flux, int rk, int steps, bool monitor, cudaStream_t stream);
 // The tile-staged stage kernel: one CTA per tile of kTile elements (each
 // interior flux once per tile, traces shared in shared memory), `ctas` CTAs
 // per launch looping over the tiles (0 = one CTA per tile).  `order` 1 or 2,
@@ -275,7 +300,8 @@ bool tiled_fits(int prec, int order, int flux, int max_halo, int tile);
 // resident CTAs per SM of the tiled stage kernel (order 3: mixed pack) for
 // tiles of `tile` elements
 int tiled_max_ctas_per_sm(int prec, int order, int nq, int flux, int max_halo, int tile = kTile);
-int sm_count();  // SMs of the current device
+int sm_count();       // SMs of the current device
+size_t smem_limit();  // dynamic shared memory a CTA may use
 // TVB limiter over tiles; flags[solve] (may be null: all on) enables it per
 // solve, solves whose control block (ctl may be null) says done are skipped,
 // and tiles whose tile_flags entry (may be null) is 0 -- the stage kernel

@@ -141,22 +141,98 @@ __device__ __forceinline__ void hllc_flux(const double uL[4], const double uR[4]
     f[2] = fma(c, fma(d, ny, u2), fma(u2, q, mul_(p, ny)));
     f[3] = fma(c, fma(d, SM, ep), mul_(ep, q));
 }
-// LLF coefficient from the average of the two cell means
-// (src/kernelfunctions.cu:370-387), scaled by the edge length.
-__device__ __forceinline__ double llf_alpha(const double mL[4], const double mR[4], double Nx, double Ny, double len,
-                                            double gamma, double gm1) {
-    double m[4];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) m[v] = mul_(0.5, add_(mL[v], mR[v]));
-    const double ir = rcp_f64(m[0]), vx = mul_(m[1], ir), vy = mul_(m[2], ir);
-    const double p = mul_(gm1, fma(-0.5, fma(m[1], vx, mul_(m[2], vy)), m[3]));
-    return fma(sqrt_f64(mul_(mul_(gamma, p), ir)), len, fabs(fma(vx, Nx, mul_(vy, Ny))));
-}
-
 // Runge-Kutta combination U^n + b ((U - U^n) + dt R) of one value; without
 // U^n, b (U + dt R).
 __device__ __forceinline__ double rk_combine(double u, double u0, double r, double dt, double b) {
     return fma(b, fma(dt, r, add_(u, -u0)), u0);
+}
+
+// The flux tasks of a tile: own traces s_tr [3 NG][2][BT], halo traces s_htr
+// [NG][2][HM] followed by the halo means (LLF), the tile's means s_mean
+// [2][BT] (LLF); NT threads.
+template <int NG, int FLUX, int BT, int NT>
+__device__ __forceinline__ void flux_tasks64(int nt, const uint16_t* s_task, const int4* s_code, const double* s_nrm,
+                                             double2* s_tr, const double2* s_mean, const double2* s_htr, int HM,
+                                             const double* s_far, double gamma) {
+    constexpr int NC = TiledLayout<double, BT>::NC;
+    const double gm1 = add_(gamma, -1.0);
+    for (int j = threadIdx.x; j < nt; j += NT) {
+        const int tkj = s_task[j];
+        const int le = tkj >> 2, k = tkj & 3;
+        const int c = reinterpret_cast<const int*>(s_code + le)[k];
+        const int kind = c & 3, se = (c >> 2) & 3, idx = c >> 4;
+        // physical normal N (|N| = edge length) and unit normal of edge k
+        const double Nx = s_nrm[(NC * k + 0) * BT + le], Ny = s_nrm[(NC * k + 1) * BT + le];
+        double len, il;
+        roots_f64(fma(Nx, Nx, mul_(Ny, Ny)), len, il);
+        const double nx = mul_(Nx, il), ny = mul_(Ny, il);
+        // the other side's values: in-tile slots, or the halo rows
+        const double2* nb = kind == EDGE_HALO ? s_htr + idx : s_tr + (size_t)2 * se * NG * BT + idx;
+        const int nld = kind == EDGE_HALO ? HM : BT;
+        double alpha = 0.0;
+        if constexpr (FLUX == RKDG_FLUX_LLF) {
+            double2 x = s_mean[le], y = s_mean[BT + le];
+            const double mL[4] = {x.x, x.y, y.x, y.y};
+            double mR[4];
+            if (kind == EDGE_BOUNDARY) {
+                ghost<double>(se, mL, s_far, nx, ny, mR);
+            } else {
+                const double2* mb = kind == EDGE_HALO ? nb + 2 * NG * HM : s_mean + idx;
+                x = mb[0], y = mb[nld];
+                mR[0] = x.x, mR[1] = x.y, mR[2] = y.x, mR[3] = y.y;
+            }
+            alpha = llf_alpha<double>(mL, mR, Nx, Ny, len, gamma, gm1);
+        }
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+            double2* slot = s_tr + 2 * (k * NG + g) * BT + le;
+            double2 x = slot[0], y = slot[BT];
+            const double uL[4] = {x.x, x.y, y.x, y.y};
+            double uR[4], f[4];
+            // the neighbour's point NG-1-g on its edge se pairs with ours
+            // (src/kernelfunctions.cu:545-549)
+            const double2* np = nb + 2 * (NG - 1 - g) * nld;
+            if (kind == EDGE_BOUNDARY) {
+                ghost<double>(se, uL, s_far, nx, ny, uR);
+            } else {
+                x = np[0], y = np[nld];
+                uR[0] = x.x, uR[1] = x.y, uR[2] = y.x, uR[3] = y.y;
+            }
+            if constexpr (FLUX == RKDG_FLUX_LLF) {
+                llf_flux(uL, uR, Nx, Ny, alpha, gm1, f);
+            } else {
+                hllc_flux(uL, uR, nx, ny, gamma, f);
+#pragma unroll
+                for (int v = 0; v < 4; ++v) f[v] = mul_(f[v], len);
+            }
+            // each slot of an edge is read by this task alone: the computing
+            // side's slot takes the flux, an in-tile neighbour's its negation
+            slot[0] = make_double2(f[0], f[1]);
+            slot[BT] = make_double2(f[2], f[3]);
+            if (kind == EDGE_IN_OWNER) {
+                double2* ns = const_cast<double2*>(np);
+                ns[0] = make_double2(-f[0], -f[1]);
+                ns[BT] = make_double2(-f[2], -f[3]);
+            }
+        }
+    }
+}
+
+// Surface term: the outward fluxes in an element's own slots.
+template <int NB, int NG, int BT>
+__device__ __forceinline__ void project64(const Tab<double>& tb, const double2* s_tr, double2 R[NB][2]) {
+#pragma unroll
+    for (int s = 0; s < 3 * NG; ++s) {
+        const double* w = tb.ephiw[s / NG][s % NG];
+        const double2 f[2] = {s_tr[2 * s * BT + threadIdx.x], s_tr[(2 * s + 1) * BT + threadIdx.x]};
+#pragma unroll
+        for (int i = 0; i < NB; ++i)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                R[i][h].x = fma(-f[h].x, w[i], R[i][h].x);
+                R[i][h].y = fma(-f[h].y, w[i], R[i][h].y);
+            }
+    }
 }
 
 // One tile, as tile_stage (stage_tiled.cuh).  Own trace slot s = k NG + g,
@@ -236,66 +312,7 @@ __device__ __forceinline__ bool tile_stage_fp64(const StageArgs& a, const TileAr
     }
 
     // ------------------------------------------------------------ phase B
-    for (int j = tid; j < nt; j += NT) {
-        const int tkj = s_task[j];
-        const int le = tkj >> 2, k = tkj & 3;
-        const int c = reinterpret_cast<const int*>(s_code + le)[k];
-        const int kind = c & 3, se = (c >> 2) & 3, idx = c >> 4;
-        // physical normal N (|N| = edge length) and unit normal of edge k
-        const double Nx = s_nrm[(NC * k + 0) * BT + le], Ny = s_nrm[(NC * k + 1) * BT + le];
-        double len, il;
-        roots_f64(fma(Nx, Nx, mul_(Ny, Ny)), len, il);
-        const double nx = mul_(Nx, il), ny = mul_(Ny, il);
-        // the other side's values: in-tile slots, or the halo rows
-        const double2* nb = kind == EDGE_HALO ? s_stg + idx : s_tr + (size_t)2 * se * NG * BT + idx;
-        const int nld = kind == EDGE_HALO ? HM : BT;
-        double alpha = 0.0;
-        if constexpr (FLUX == RKDG_FLUX_LLF) {
-            double2 x = s_mean[le], y = s_mean[BT + le];
-            const double mL[4] = {x.x, x.y, y.x, y.y};
-            double mR[4];
-            if (kind == EDGE_BOUNDARY) {
-                ghost<double>(se, mL, s_far, nx, ny, mR);
-            } else {
-                const double2* mb = kind == EDGE_HALO ? nb + 2 * NG * HM : s_mean + idx;
-                x = mb[0], y = mb[nld];
-                mR[0] = x.x, mR[1] = x.y, mR[2] = y.x, mR[3] = y.y;
-            }
-            alpha = llf_alpha(mL, mR, Nx, Ny, len, gamma, gm1);
-        }
-#pragma unroll
-        for (int g = 0; g < NG; ++g) {
-            double2* slot = s_tr + 2 * (k * NG + g) * BT + le;
-            double2 x = slot[0], y = slot[BT];
-            const double uL[4] = {x.x, x.y, y.x, y.y};
-            double uR[4], f[4];
-            // the neighbour's point NG-1-g on its edge se pairs with ours
-            // (src/kernelfunctions.cu:545-549)
-            const double2* np = nb + 2 * (NG - 1 - g) * nld;
-            if (kind == EDGE_BOUNDARY) {
-                ghost<double>(se, uL, s_far, nx, ny, uR);
-            } else {
-                x = np[0], y = np[nld];
-                uR[0] = x.x, uR[1] = x.y, uR[2] = y.x, uR[3] = y.y;
-            }
-            if constexpr (FLUX == RKDG_FLUX_LLF) {
-                llf_flux(uL, uR, Nx, Ny, alpha, gm1, f);
-            } else {
-                hllc_flux(uL, uR, nx, ny, gamma, f);
-#pragma unroll
-                for (int v = 0; v < 4; ++v) f[v] = mul_(f[v], len);
-            }
-            // each slot of an edge is read by this task alone: the computing
-            // side's slot takes the flux, an in-tile neighbour's its negation
-            slot[0] = make_double2(f[0], f[1]);
-            slot[BT] = make_double2(f[2], f[3]);
-            if (kind == EDGE_IN_OWNER) {
-                double2* ns = const_cast<double2*>(np);
-                ns[0] = make_double2(-f[0], -f[1]);
-                ns[BT] = make_double2(-f[2], -f[3]);
-            }
-        }
-    }
+    flux_tasks64<NG, FLUX, BT, BT>(nt, s_task, s_code, s_nrm, s_tr, s_mean, s_stg, HM, s_far, gamma);
     __syncthreads();  // fluxes complete, halo traces read: the staging area takes the next tile's rows
     if (tid == 0 && nxt < ntiles) {
         fence_proxy_async();
@@ -304,18 +321,7 @@ __device__ __forceinline__ bool tile_stage_fp64(const StageArgs& a, const TileAr
 
     // ------------------------------------------------------------ phase C
     // every own slot now holds the outward flux of its edge point
-#pragma unroll
-    for (int s = 0; s < 3 * NG; ++s) {
-        const double* w = tb.ephiw[s / NG][s % NG];
-        const double2 f[2] = {s_tr[2 * s * BT + tid], s_tr[(2 * s + 1) * BT + tid]};
-#pragma unroll
-        for (int i = 0; i < NB; ++i)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                R[i][h].x = fma(-f[h].x, w[i], R[i][h].x);
-                R[i][h].y = fma(-f[h].y, w[i], R[i][h].y);
-            }
-    }
+    project64<NB, NG, BT>(tb, s_tr, R);
 
     double2* Uout = static_cast<double2*>(a.Unew) + ee;
     if (MODE == MODE_RESIDUAL) {

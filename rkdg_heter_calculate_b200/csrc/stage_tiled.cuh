@@ -99,21 +99,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint64
     return false;
 }
 
-// Self-test of the bounded wait: one thread arms an mbarrier for 16 bytes
-// that no copy ever delivers and waits on it with the given limit; out[0] =
-// 1 if the wait gave up, out[1] = nanoseconds waited.  Nothing is in flight
-// when it returns.
-__global__ void wait_selftest_kernel(uint64_t limit_ns, unsigned long long* out) {
-    __shared__ __align__(8) uint64_t bar;
-    if (threadIdx.x != 0) return;
-    mbar_init(&bar, 1);
-    mbar_expect_tx(&bar, 16);
-    const uint64_t t0 = global_ns();
-    const bool ok = mbar_wait(&bar, 0, limit_ns);
-    out[0] = ok ? 0ull : 1ull;
-    out[1] = global_ns() - t0;
-}
-
 // Shared memory of one CTA: the work area (edge normals, edge codes, flux
 // tasks, own traces and means, as 4-vectors), sized for the largest tile
 // layout the kernel dispatches (P1 tiles of a mixed pack use a prefix),
@@ -293,11 +278,35 @@ struct TilePre {
     double det;                         // det J^-1 = 1 / (2 area)
     int2 hh[3];
 };
+// The geometry of TilePre, and the edge normals into s_nrm, the element's
+// entry of [3][NC][BT] (or null).
+template <int BT>
+__device__ __forceinline__ void tile_geom(const double2 r0, const double2 r1, float* s_nrm, TilePre<float>& t) {
+    using Real = float;
+    constexpr int NC = TiledLayout<Real, BT>::NC;
+    // edge normals N_k (length = edge length; N_k / area = 2(r0 + r1), -2 r0,
+    // -2 r1) from the FP64 J^-1 rows, kept in the working precision.  The
+    // residual is accumulated scaled by 2 area (= 1 / det J^-1): the volume
+    // term through 2 area J^-1 = (-N_1; -N_2), the surface term through the
+    // table 2 w_g psi_i, and the factor det J^-1 applied once in the update.
+    t.det = fma(r0.x, r1.y, -mul_(r0.y, r1.x));
+    t.inv_area = (Real)(2.0 * t.det);
+    // from the rounded J^-1 rows (a few ulp, without an FP64 reciprocal)
+    const Real area2 = rcp_((Real)t.det);
+    const Real ax = (Real)r0.x, ay = (Real)r0.y, bx = (Real)r1.x, by = (Real)r1.y;
+    const Real cx[3] = {add_(ax, bx), -ax, -bx}, cy[3] = {add_(ay, by), -ay, -by};
+    Real Nx[3], Ny[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        Nx[k] = mul_(cx[k], area2), Ny[k] = mul_(cy[k], area2);
+        if (s_nrm) s_nrm[(NC * k + 0) * BT] = Nx[k], s_nrm[(NC * k + 1) * BT] = Ny[k];
+    }
+    t.j00 = -Nx[1], t.j01 = -Ny[1], t.j10 = -Nx[2], t.j11 = -Ny[2];
+}
 template <typename Real, int BT>
 __device__ __forceinline__ TilePre<Real> tile_pre(const StageArgs& a, const TileArgs& ta, const int4 d0,
                                                   const int4 d1, const double2 r0, const double2 r1,
                                                   const int4 code, unsigned char* smem_raw) {
-    constexpr int NC = TiledLayout<Real, BT>::NC;
     const int tid = threadIdx.x;
     TilePre<Real> t;
     t.rs = ref_state(a.ref32, d0.z);
@@ -313,27 +322,7 @@ __device__ __forceinline__ TilePre<Real> tile_pre(const StageArgs& a, const Tile
         if (h < nt) s_task[h] = __ldg(ta.task + t0 + h);
     }
     s_code[tid] = code;
-    // edge normals N_k (length = edge length; N_k / area = 2(r0 + r1), -2 r0,
-    // -2 r1) from the FP64 J^-1 rows, kept in the working precision.  The
-    // residual is accumulated scaled by 2 area (= 1 / det J^-1): the volume
-    // term through 2 area J^-1 = (-N_1; -N_2), the surface term through the
-    // table 2 w_g psi_i, and the factor det J^-1 applied once in the update.
-    Real* s_nrm = reinterpret_cast<Real*>(smem_raw);  // [3][NC][BT] Nx, Ny
-    t.det = r0.x * r1.y - r0.y * r1.x;
-    t.inv_area = (Real)(2.0 * t.det);
-    // FP64 forms them in FP64; FP32 from the rounded J^-1 rows (a few ulp,
-    // without the FP64 reciprocal)
-    const Real area2 = rcp_((Real)t.det);
-    const Real ax = (Real)r0.x, ay = (Real)r0.y, bx = (Real)r1.x, by = (Real)r1.y;
-    const Real cx[3] = {ax + bx, -ax, -bx}, cy[3] = {ay + by, -ay, -by};
-    Real Nx[3], Ny[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        Nx[k] = cx[k] * area2, Ny[k] = cy[k] * area2;
-        s_nrm[(NC * k + 0) * BT + tid] = Nx[k];
-        s_nrm[(NC * k + 1) * BT + tid] = Ny[k];
-    }
-    t.j00 = -Nx[1], t.j01 = -Ny[1], t.j10 = -Nx[2], t.j11 = -Ny[2];
+    tile_geom<BT>(r0, r1, reinterpret_cast<Real*>(smem_raw) + tid, t);
     return t;
 }
 
@@ -347,6 +336,132 @@ __device__ __forceinline__ void load_edge_table(const T (*g)[3 * kMaxNG * kMaxNB
     for (int x = threadIdx.x; x < n; x += BT) s[0][x] = __ldg(&g[ORD == 1 ? P1 : cfg_index(NQ2, 3)][x]);
     if constexpr (ORD == 3)
         for (int x = threadIdx.x; x < 3 * 2 * 3; x += BT) s[1][x] = __ldg(&g[P1][x]);
+}
+
+// Volume term of rows 1.. from an element's modes u: flux deviations through
+// the rows of 2 area J^-1.  The quadrature loop is unrolled by two only (a
+// smaller body keeps the instruction cache warm across the CTAs on an SM;
+// full unrolling is 2 % slower, none 1 %).  psi_0 is one at every point and
+// psi_1 (a function of xi alone) has no eta-derivative term.
+template <int NB, int NQ>
+__device__ __forceinline__ void volume32(const Tab2& t2, const float u[NB][4], const RefState<float>& rs, float j00,
+                                         float j01, float j10, float j11, float gm1, float R[NB][4]) {
+#pragma unroll 2
+    for (int q = 0; q < NQ; ++q) {
+        float w[4], fx[4], fy[4];
+        comb_rows<NB>(t2.vphi[q], u, lo2(u[0]), hi2(u[0]), w);
+        const DevPrims<float> pw = dev_prims(w, rs, gm1);
+        dev_flux(w, pw, rs, j00, j01, fx);
+        dev_flux(w, pw, rs, j10, j11, fy);
+        acc_rows<1, NB>(R, fx, t2.vdxi[q]);
+        acc_rows<2, NB>(R, fy, t2.veta[q]);
+    }
+}
+
+// The flux tasks of a tile: own traces s_tr [3][NG][BT], halo traces s_htr
+// [NG][HM] followed by the halo means (LLF), the tile's means s_mean (LLF).
+template <int NG, int FLUX, int BT, int NT>
+__device__ __forceinline__ void flux_tasks32(int nt, const uint16_t* s_task, const int4* s_code, const float* s_nrm,
+                                             Vec4<float>* s_tr, const Vec4<float>* s_mean, Vec4<float>* s_htr, int HM,
+                                             const RefState<float>& rs, float gamma) {
+    using Real = float;
+    using V4 = Vec4<float>;
+    constexpr int NC = TiledLayout<Real, BT>::NC;
+    constexpr bool MEANS = FLUX == RKDG_FLUX_LLF;
+    const Real gm1 = add_(gamma, -1.0f);
+    const Real far[4] = {rs.rho, rs.mx, rs.my, rs.E};
+    for (int j = threadIdx.x; j < nt; j += NT) {
+        const int tkj = s_task[j];
+        const int le = tkj >> 2, k = tkj & 3;
+        const int c = reinterpret_cast<const int*>(s_code + le)[k];
+        const int kind = c & 3, se = (c >> 2) & 3, idx = c >> 4;
+        // physical normal N (|N| = edge length) and unit normal of edge k
+        const Real Nx = s_nrm[(NC * k + 0) * BT + le], Ny = s_nrm[(NC * k + 1) * BT + le];
+        Real len, il;
+        lengths_(fma(Nx, Nx, mul_(Ny, Ny)), len, il);
+        const Real nx = mul_(Nx, il), ny = mul_(Ny, il);
+        Real alpha = Real(0);
+        if constexpr (MEANS) {
+            Real mL[4], mR[4];
+            get4(s_mean + le, mL);
+            if (kind == EDGE_BOUNDARY) ghost<Real>(se, mL, far, nx, ny, mR);
+            else get4(kind == EDGE_HALO ? s_htr + NG * HM + idx : s_mean + idx, mR);
+            alpha = llf_alpha<Real>(mL, mR, Nx, Ny, len, gamma, gm1);
+        }
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+            Real uL[4], uR[4];
+            V4* slot = s_tr + (k * NG + g) * BT + le;
+            get4(slot, uL);
+            // the neighbour's point NG-1-g on its edge se pairs with ours
+            // (src/kernelfunctions.cu:545-549)
+            V4* nslot = kind == EDGE_HALO ? s_htr + (NG - 1 - g) * HM + idx : s_tr + (se * NG + NG - 1 - g) * BT + idx;
+            if (kind == EDGE_BOUNDARY) ghost_dev<Real>(se, uL, rs, nx, ny, uR);
+            else get4(nslot, uR);
+            Real fh[4], fn[4];  // the flux out of this side and into the neighbour
+            if (FLUX == RKDG_FLUX_LLF) {
+                Real fL[4], fR[4];
+                dev_flux(uL, dev_prims(uL, rs, gm1), rs, Nx, Ny, fL);
+                dev_flux(uR, dev_prims(uR, rs, gm1), rs, Nx, Ny, fR);
+                const float2 na = make_float2(-alpha, -alpha);
+                const float2 tl = f2fma(na, f2sub(lo2(uR), lo2(uL)), f2add(lo2(fL), lo2(fR)));
+                const float2 th = f2fma(na, f2sub(hi2(uR), hi2(uL)), f2add(hi2(fL), hi2(fR)));
+                const float2 hp = make_float2(0.5f, 0.5f), hn = make_float2(-0.5f, -0.5f);
+                set4(fh, f2mul(hp, tl), f2mul(hp, th));
+                set4(fn, f2mul(hn, tl), f2mul(hn, th));
+            } else {
+                Real f[4];
+                hllc_dev(uL, uR, nx, ny, gamma, rs, f);
+                const float2 l = make_float2(len, len), nl = make_float2(-len, -len);
+                set4(fh, f2mul(lo2(f), l), f2mul(hi2(f), l));
+                set4(fn, f2mul(lo2(f), nl), f2mul(hi2(f), nl));
+            }
+            // each slot of an edge is read by this task alone: the computing
+            // side's slot takes the flux, an in-tile neighbour's its negation
+            put4(slot, fh);
+            if (kind == EDGE_IN_OWNER) put4(nslot, fn);
+        }
+    }
+}
+
+// Surface term: the outward fluxes in an element's own slots.
+template <int NB, int NG, int BT>
+__device__ __forceinline__ void project32(const Tab2& t2, const Vec4<float>* s_tr, float R[NB][4]) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+            float f[4];
+            get4(s_tr + (k * NG + g) * BT + threadIdx.x, f);
+            acc_rows<0, NB>(R, f, t2.nephiw[k][g]);
+        }
+}
+
+// Runge-Kutta update of one row: U^n + b ((U - U^n) + dt R) (a U^n + b (U +
+// dt L) with a + b = 1 exactly: 1/3 and 2/3 both round up in FP32, and a
+// scale of 1 + 3e-8 per step would accumulate), or b (U + dt R) in a first
+// stage.
+__device__ __forceinline__ void update_row32(const float u[4], const float u0[4], float dt, float b, float r[4]) {
+    const float2 dt2 = make_float2(dt, dt), b2 = make_float2(b, b);
+    set4(r, f2fma(b2, f2fma(dt2, lo2(r), f2sub(lo2(u), lo2(u0))), lo2(u0)),
+         f2fma(b2, f2fma(dt2, hi2(r), f2sub(hi2(u), hi2(u0))), hi2(u0)));
+}
+__device__ __forceinline__ void update_row32(const float u[4], float dt, float b, float r[4]) {
+    const float2 dt2 = make_float2(dt, dt), b2 = make_float2(b, b);
+    set4(r, f2mul(b2, f2fma(dt2, lo2(r), lo2(u))), f2mul(b2, f2fma(dt2, hi2(r), hi2(u))));
+}
+// RKDG_FP32C: the mean's update in FP64 from its high and low parts (h, l;
+// U^n's h0, l0, zero in a first stage), split again, so that the mean's
+// storage rounding does not accumulate over the stages.
+__device__ __forceinline__ void update_mean32c(const float h[4], const float l[4], const float h0[4], const float l0[4],
+                                               double dt, double b, float r[4], float low[4]) {
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+        const double m = add_((double)h[v], (double)l[v]), m0 = add_((double)h0[v], (double)l0[v]);
+        const double y = fma(b, fma(dt, (double)r[v], add_(m, -m0)), m0);
+        r[v] = (float)y;
+        low[v] = (float)add_(y, -(double)r[v]);
+    }
 }
 
 // Returns, when the stage is followed by the TVB limiter (a.tile_flags set),
@@ -373,7 +488,7 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
     // Each halo thread writes only its own entry, after it has read the rows
     // there.
     V4* s_htr = reinterpret_cast<V4*>(stg);
-    V4* s_hmean = s_htr + NG * HM;
+    V4* s_hmean = s_htr + NG * HM;  // (LLF)
     const Tab2& t2 = c_tab_f2[CFG];   // paired tables of the lane-pair arithmetic
     const int sid = d0.z;
     StepCtl* ctl = a.ctl + sid;
@@ -418,29 +533,14 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
         {
             Real mfull[4];
 #pragma unroll
-            for (int v = 0; v < 4; ++v) mfull[v] = u[0][v] + far[v];  // the cell mean itself
+            for (int v = 0; v < 4; ++v) mfull[v] = add_(u[0][v], far[v]);  // the cell mean itself
             if constexpr (MEANS) put4(s_mean + tid, mfull);
         }
 #pragma unroll
         for (int i = 0; i < NB; ++i)
 #pragma unroll
             for (int v = 0; v < 4; ++v) R[i][v] = Real(0);
-        // the quadrature loop is unrolled by two only (a smaller body keeps
-        // the instruction cache warm across the CTAs on an SM; full unrolling
-        // is 2 % slower, none 1 %).  psi_0 is one at every point and psi_1 (a
-        // function of xi alone) has no eta-derivative term.
-#pragma unroll 2
-        for (int q = 0; q < NQ; ++q) {
-            Real w[4];
-            comb_rows<NB>(t2.vphi[q], u, lo2(u[0]), hi2(u[0]), w);
-            Real fx[4], fy[4];
-            // flux deviations through the rows of 2 area J^-1
-            const DevPrims<Real> pw = dev_prims(w, rs, gm1);
-            dev_flux(w, pw, rs, j00, j01, fx);
-            dev_flux(w, pw, rs, j10, j11, fy);
-            acc_rows<1, NB>(R, fx, t2.vdxi[q]);
-            acc_rows<2, NB>(R, fy, t2.veta[q]);
-        }
+        volume32<NB, NQ>(t2, u, rs, j00, j01, j10, j11, gm1, R);
 #pragma unroll
         for (int k = 0; k < 3; ++k)
 #pragma unroll
@@ -467,7 +567,7 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
                 if constexpr (MEANS) {
                     Real mfull[4];
 #pragma unroll
-                    for (int v = 0; v < 4; ++v) mfull[v] = un[0][v] + far[v];
+                    for (int v = 0; v < 4; ++v) mfull[v] = add_(un[0][v], far[v]);
                     put4(s_hmean + h, mfull);
                 }
                 const int he = hh[r].y;
@@ -489,71 +589,7 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
     prefetch_ahead<Real, BT>(a, ta, nxt, ntiles);
 
     // ------------------------------------------------------------ phase B
-    {
-        for (int j = tid; j < nt; j += BT) {
-            const int tkj = s_task[j];
-            const int le = tkj >> 2, k = tkj & 3;
-            const int c = reinterpret_cast<const int*>(s_code + le)[k];
-            const int kind = c & 3, se = (c >> 2) & 3, idx = c >> 4;
-            // physical normal N (|N| = edge length) and unit normal of edge k
-            const Real Nx = s_nrm[(NC * k + 0) * BT + le], Ny = s_nrm[(NC * k + 1) * BT + le];
-            Real len, il;
-            lengths_(Nx * Nx + Ny * Ny, len, il);
-            const Real nx = Nx * il, ny = Ny * il;
-            Real mL[4], mR[4];
-            if constexpr (MEANS) {
-                get4(s_mean + le, mL);
-                if (kind == EDGE_BOUNDARY) ghost<Real>(se, mL, far, nx, ny, mR);
-                else get4(kind == EDGE_HALO ? s_hmean + idx : s_mean + idx, mR);
-            }
-            Real alpha = Real(0);
-            if constexpr (FLUX == RKDG_FLUX_LLF) {
-                // LLF coefficient from the average of the two cell means
-                // (src/kernelfunctions.cu:370-387), scaled by the edge length
-                Real rho = Real(0.5) * (mL[0] + mR[0]);
-                Real ir = rcp_(rho);
-                Real vx = Real(0.5) * (mL[1] + mR[1]) * ir;
-                Real vy = Real(0.5) * (mL[2] + mR[2]) * ir;
-                Real E = Real(0.5) * (mL[3] + mR[3]);
-                Real p = gm1 * (E - Real(0.5) * rho * (vx * vx + vy * vy));
-                alpha = fabs(vx * Nx + vy * Ny) + sqrt_(gamma * p * ir) * len;
-            }
-#pragma unroll
-            for (int g = 0; g < NG; ++g) {
-                Real uL[4], uR[4];
-                V4* slot = s_tr + (k * NG + g) * BT + le;
-                get4(slot, uL);
-                // the neighbour's point NG-1-g on its edge se pairs with ours
-                // (src/kernelfunctions.cu:545-549)
-                V4* nslot = kind == EDGE_HALO ? s_htr + (NG - 1 - g) * HM + idx : s_tr + (se * NG + NG - 1 - g) * BT + idx;
-                if (kind == EDGE_BOUNDARY) ghost_dev<Real>(se, uL, rs, nx, ny, uR);
-                else get4(nslot, uR);
-                Real fh[4], fn[4];  // the flux out of this side and into the neighbour
-                if (FLUX == RKDG_FLUX_LLF) {
-                    Real fL[4], fR[4];
-                    dev_flux(uL, dev_prims(uL, rs, gm1), rs, Nx, Ny, fL);
-                    dev_flux(uR, dev_prims(uR, rs, gm1), rs, Nx, Ny, fR);
-                    const float2 na = make_float2(-alpha, -alpha);
-                    const float2 tl = f2fma(na, f2sub(lo2(uR), lo2(uL)), f2add(lo2(fL), lo2(fR)));
-                    const float2 th = f2fma(na, f2sub(hi2(uR), hi2(uL)), f2add(hi2(fL), hi2(fR)));
-                    const float2 hp = make_float2(0.5f, 0.5f), hn = make_float2(-0.5f, -0.5f);
-                    set4(fh, f2mul(hp, tl), f2mul(hp, th));
-                    set4(fn, f2mul(hn, tl), f2mul(hn, th));
-                } else {
-                    Real f[4];
-                    hllc_dev<Real>(uL, uR, nx, ny, gamma, rs, f);
-                    const float2 l = make_float2(len, len), nl = make_float2(-len, -len);
-                    set4(fh, f2mul(lo2(f), l), f2mul(hi2(f), l));
-                    set4(fn, f2mul(lo2(f), nl), f2mul(hi2(f), nl));
-                }
-                // each slot of an edge is read by this task alone: the
-                // computing side's slot takes the flux, an in-tile
-                // neighbour's slot its negation
-                put4(slot, fh);
-                if (kind == EDGE_IN_OWNER) put4(nslot, fn);
-            }
-        }
-    }
+    flux_tasks32<NG, FLUX, BT, BT>(nt, s_task, s_code, s_nrm, s_tr, s_mean, s_htr, HM, rs, gamma);
     __syncthreads();  // fluxes complete, halo traces read: the staging area takes the next tile's rows
     if (tid == 0 && nxt < ntiles) {
         fence_proxy_async();
@@ -562,14 +598,7 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
 
     // ------------------------------------------------------------ phase C
     // every own slot now holds the outward flux of its edge point
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-#pragma unroll
-        for (int g = 0; g < NG; ++g) {
-            Real f[4];
-            get4(s_tr + (k * NG + g) * BT + tid, f);
-            acc_rows<0, NB>(R, f, t2.nephiw[k][g]);
-        }
+    project32<NB, NG, BT>(t2, s_tr, R);
 
     Real* __restrict__ Uout = static_cast<Real*>(a.Unew);
     if (MODE == MODE_RESIDUAL) {
@@ -582,36 +611,21 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
         return false;
     }
     const double dtd = *s_dt;
-    // a U^n + b (U + dt L) as U^n + b ((U - U^n) + dt L): a + b = 1 holds
-    // exactly (1/3 and 2/3 both round up in FP32, and a scale of 1 + 3e-8
-    // per step would accumulate into the state); L = det J^-1 R
-    const Real dt = (Real)(dtd * det), cb = (Real)a.b;
+    const Real dt = (Real)mul_(dtd, det), cb = (Real)a.b;
     Real u0m[4] = {Real(0), Real(0), Real(0), Real(0)};
     // RKDG_FP32C (comp): row 0 is updated in FP64 below, not here
     constexpr bool comp = (MODE & MODE_STAGE_COMP) != 0;
-    {
-        load_state<Real, NB>(U, a.ld, ee, u);  // stored values (L2 hit)
-        if (a.U0 != nullptr) {
-            Real u0[NB][4];
-            load_state<Real, NB>(static_cast<const Real*>(a.U0), a.ld, ee, u0);
-            const float2 dt2 = make_float2(dt, dt), cb2 = make_float2(cb, cb);
+    load_state<Real, NB>(U, a.ld, ee, u);  // stored values (L2 hit)
+    if (a.U0 != nullptr) {
+        Real u0[NB][4];
+        load_state<Real, NB>(static_cast<const Real*>(a.U0), a.ld, ee, u0);
 #pragma unroll
-            for (int i = 0; i < NB; ++i) {
-                const float2 l = f2fma(cb2, f2fma(dt2, lo2(R[i]), f2sub(lo2(u[i]), lo2(u0[i]))), lo2(u0[i]));
-                const float2 h = f2fma(cb2, f2fma(dt2, hi2(R[i]), f2sub(hi2(u[i]), hi2(u0[i]))), hi2(u0[i]));
-                if (i > 0 || !comp) set4(R[i], l, h);
-            }
+        for (int i = comp ? 1 : 0; i < NB; ++i) update_row32(u[i], u0[i], dt, cb, R[i]);
 #pragma unroll
-            for (int v = 0; v < 4; ++v) u0m[v] = u0[0][v];
-        } else {
-            const float2 dt2 = make_float2(dt, dt), cb2 = make_float2(cb, cb);
+        for (int v = 0; v < 4; ++v) u0m[v] = u0[0][v];
+    } else {
 #pragma unroll
-            for (int i = 0; i < NB; ++i) {
-                const float2 l = f2mul(cb2, f2fma(dt2, lo2(R[i]), lo2(u[i])));
-                const float2 h = f2mul(cb2, f2fma(dt2, hi2(R[i]), hi2(u[i])));
-                if (i > 0 || !comp) set4(R[i], l, h);
-            }
-        }
+        for (int i = comp ? 1 : 0; i < NB; ++i) update_row32(u[i], dt, cb, R[i]);
     }
     if constexpr (comp) {
         // RKDG_FP32C: the cell mean is the unevaluated sum of its stored high
@@ -622,25 +636,12 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
         // accumulate over the stages.
         if (active) store_rows<Real, 1, NB>(Uout, a.ld, e, R);
         const size_t lr = (size_t)a.lo_row * a.ld;
-        // the high parts: the stage input's and U^n's row 0 as loaded for
-        // the update above (U^n's is zero in a first stage)
-        const float4 h = make_float4(u[0][0], u[0][1], u[0][2], u[0][3]);
-        const float4 h0 = make_float4(u0m[0], u0m[1], u0m[2], u0m[3]);
         const float4 l = __ldg(reinterpret_cast<const float4*>(a.U) + lr + ee);
         float4 l0 = make_float4(0.f, 0.f, 0.f, 0.f);
         if (a.U0 != nullptr) l0 = __ldg(reinterpret_cast<const float4*>(a.U0) + lr + ee);
-        const double dtdet = dtd * det;
-        const float hv[4] = {h.x, h.y, h.z, h.w}, lv[4] = {l.x, l.y, l.z, l.w};
-        const float h0v[4] = {h0.x, h0.y, h0.z, h0.w}, l0v[4] = {l0.x, l0.y, l0.z, l0.w};
+        const float lv[4] = {l.x, l.y, l.z, l.w}, l0v[4] = {l0.x, l0.y, l0.z, l0.w};
         float nl[4];
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const double m = (double)hv[v] + (double)lv[v], m0 = (double)h0v[v] + (double)l0v[v];
-            const double y = m0 + a.b * ((m - m0) + dtdet * (double)R[0][v]);
-            const float yh = (float)y;
-            R[0][v] = yh;
-            nl[v] = (float)(y - (double)yh);
-        }
+        update_mean32c(u[0], lv, u0m, l0v, mul_(dtd, det), a.b, R[0], nl);
         if (active) {
             reinterpret_cast<float4*>(a.Unew)[e] = make_float4(R[0][0], R[0][1], R[0][2], R[0][3]);
             reinterpret_cast<float4*>(a.Unew)[lr + e] = make_float4(nl[0], nl[1], nl[2], nl[3]);
@@ -660,17 +661,17 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
             bool bad;
             Real m[4], len[3];
 #pragma unroll
-            for (int v = 0; v < 4; ++v) m[v] = R[0][v] + far[v];
+            for (int v = 0; v < 4; ++v) m[v] = add_(R[0][v], far[v]);
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 const Real Nx = s_nrm[(NC * k + 0) * BT + tid], Ny = s_nrm[(NC * k + 1) * BT + tid];
-                len[k] = sqrt_(Nx * Nx + Ny * Ny);
+                len[k] = sqrt_(fma(Nx, Nx, mul_(Ny, Ny)));
             }
             wv = (Real)wave_of<Real>(m, gamma, len, inv_area, bad);
             if (bad) atomicOr(&ctl->error, 1);
             if (a.monitor) {
-                m0 = fabs(R[0][0] - u0m[0]);
-                m1 = fabs(R[0][3] - u0m[3]);
+                m0 = fabs(add_(R[0][0], -u0m[0]));
+                m1 = fabs(add_(R[0][3], -u0m[3]));
             }
         }
         wv = warp_max(wv);
@@ -692,7 +693,7 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
         // J^-1: the columns of J are (j11, -j10) and (-j01, j00))
         Real mean[4], tmax = Real(0);
 #pragma unroll
-        for (int v = 0; v < 4; ++v) mean[v] = R[0][v] + far[v];
+        for (int v = 0; v < 4; ++v) mean[v] = add_(R[0][v], far[v]);
 #pragma unroll
         for (int k = 0; k < 3; ++k)
 #pragma unroll

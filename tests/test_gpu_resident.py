@@ -1,0 +1,102 @@
+"""Whole steps in one launch (csrc/resident.cuh) against the same steps through
+the stage kernels: a context made as one partition that owns the whole mesh
+keeps the stage kernels and the caller's order, so with reorder=False both run
+the same tiles and must give the same bits, whatever the method.  Sizes: one
+tile, a ragged second one, the most tiles that run with 256 threads each (and
+one more), several launches' worth of steps (64 per launch), landing on a final
+time, and the residual history, which needs a launch per step."""
+import numpy as np
+import pytest
+
+from rkdg_heter_calculate_b200 import CUDARkdgSolver, meshgen, vortex
+
+pytestmark = pytest.mark.gpu
+
+FAR = (1.0, 1.0, 1.0, 3.5)
+
+
+def ordered(mesh):
+    return meshgen.permute(mesh, meshgen.locality_order(mesh))
+
+
+def start(mesh, nb, far, kind):
+    if kind == "vortex":
+        return vortex.project_native(mesh, lambda X, Y: vortex.exact(X, Y, 0.0, 5.0, 1.4, 1.0, 1.0), nb, n=3)
+    U = np.zeros((4, nb, mesh.ntri))  # a jump that the limiter acts on
+    c = mesh.coords().mean(axis=1)
+    scale = np.where(c[:, 0] < np.median(c[:, 0]), 1.0, 1.6)
+    for v in range(4):
+        U[v, 0] = far[v] * scale
+    return U
+
+
+def both(mesh, U, far, steps, t_final=0.0, **kw):
+    out = []
+    for whole in (None, mesh.ntri):
+        s = CUDARkdgSolver(mesh, farfield=far, reorder=False, n_owned=whole, **kw)
+        s.setFreedom(U, basis="native")
+        reached = s.advance(steps, t_final=t_final)
+        monitored = s.step()
+        out.append((s.copyFreedomToHost(basis="native"), reached, s.time(), monitored[0], tuple(monitored[1])))
+        s.close()
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    assert np.isfinite(out[0][0]).all()
+    assert out[0][1:] == out[1][1:]
+    return out[0]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32", "fp32c"])
+@pytest.mark.parametrize("order,nq,flux,limiter,rk", [(2, 7, "llf", None, 3), (2, 6, "hllc", None, 3),
+                                                      (1, 3, "llf", None, 2), (1, 3, "hllc", "tvb", 3),
+                                                      (2, 6, "llf", "tvb", 3)])
+def test_resident_equals_stage_kernels(precision, order, nq, flux, limiter, rk):
+    kw = dict(order=order, nq=nq, ng=2 if order == 1 else 3, flux=flux, limiter=limiter, rk=rk, precision=precision,
+              cfl=0.15)
+    nb = 3 if order == 1 else 6
+    for n, steps in ((8, 3), (9, 70), (25, 20)):  # 128, 162 and 1250 triangles
+        mesh = ordered(meshgen.periodic_structured(n, n, jitter=0.15, seed=n))
+        both(mesh, start(mesh, nb, FAR, "vortex"), FAR, steps, **kw)
+    # boundaries of every kind; a jump in the state where the limiter is on
+    mesh = ordered(meshgen.channel(40, 16))
+    far = (1.4, 4.2, 0.0, 8.8)
+    both(mesh, start(mesh, nb, far, "jump"), far, 10, **kw)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("n", [97, 98, 137])  # 148, 151 and 294 tiles
+def test_resident_at_the_edges_of_its_forms(precision, n):
+    mesh = ordered(meshgen.periodic_structured(n, n, jitter=0.15, seed=3))
+    both(mesh, start(mesh, 6, FAR, "vortex"), FAR, 5, order=2, nq=6, ng=3, flux="hllc", precision=precision, cfl=0.2)
+
+
+def test_resident_final_time_and_history(tmp_path):
+    mesh = ordered(meshgen.periodic_structured(20, 20, jitter=0.15, seed=2))
+    U = start(mesh, 6, FAR, "vortex")
+    kw = dict(order=2, nq=6, ng=3, flux="hllc", precision="fp64", cfl=0.2)
+    _, (t, steps), _, _, _ = both(mesh, U, FAR, 1000, t_final=0.25, **kw)
+    assert t == 0.25 and 64 < steps < 1000
+    text = []
+    for whole in (None, mesh.ntri):
+        path = tmp_path / f"history_{whole}"
+        s = CUDARkdgSolver(mesh, farfield=FAR, reorder=False, n_owned=whole, **kw)
+        s.setFreedom(U, basis="native")
+        s.setResidualLog(str(path))
+        s.advance(7)
+        s.setResidualLog(None)
+        text.append(path.read_text())
+        s.close()
+    assert text[0] == text[1] and len(text[0].splitlines()) == 8
+
+
+def test_resident_reports_a_non_physical_state():
+    from rkdg_heter_calculate_b200.capi import RkdgError
+
+    mesh = ordered(meshgen.periodic_structured(20, 20, jitter=0.15, seed=2))
+    U = start(mesh, 6, FAR, "vortex")
+    U[3, 0, 17] = -1.0
+    s = CUDARkdgSolver(mesh, farfield=FAR, order=2, nq=6, ng=3, flux="hllc", cfl=0.2)
+    s.setFreedom(U, basis="native")
+    with pytest.raises(RkdgError) as e:
+        s.advance(5)
+    assert e.value.code == 4
+    s.close()
