@@ -148,48 +148,76 @@ void coeffs(int rk, int s, double& a, double& c) {
     else a = 1.0 / 3.0, c = 2.0 / 3.0;
 }
 
-// One stage over every tile of the pack: one launch of the kernel for the
-// pack's orders, or in tile order 2 (a mixed pack) the P2 tiles with the
-// P2 kernel on the batch's stream and the P1 tiles with the P1 kernel (more
-// resident CTAs per SM) on a second stream forked from it and joined after
-// them.  A tile's arithmetic is the same in every kernel that runs it.
-void launch_pack_stage(rkdg_batch* b, const StageArgs& a) {
-    if (b->tile_order != 2 || b->ord != 3) {
-        launch_stage(a, b->tiles, b->ord, b->p.nq, b->p.flux, kprec(b), b->ctas, b->stream);
-        return;
-    }
-    TileArgs t2 = b->tiles, t1 = b->tiles;
-    t2.ntiles = b->n2tiles;
-    t1.desc = b->tdesc + 2 * (size_t)b->n2tiles;
-    t1.ntiles = b->ntiles - b->n2tiles;
+// In tile order 2 a mixed pack runs as two chains: the P2 tiles with the P2
+// kernel on the batch's stream and the P1 tiles with the P1 kernel (more
+// resident CTAs per SM) on a second one.  A tile's arithmetic is the same in
+// every kernel that runs it.
+bool two_chains(const rkdg_batch* b) { return b->tile_order == 2 && b->ord == 3; }
+
+void fork(rkdg_batch* b) {
     RKDG_CUDA_TRY(cudaEventRecord(b->ev_fork, b->stream));
     RKDG_CUDA_TRY(cudaStreamWaitEvent(b->stream2, b->ev_fork, 0));
-    if (t2.ntiles > 0) launch_stage(a, t2, 2, b->p.nq, b->p.flux, kprec(b), b->ctas, b->stream);
-    if (t1.ntiles > 0) launch_stage(a, t1, 1, b->p.nq, b->p.flux, kprec(b), b->ctas, b->stream2);
+}
+void join(rkdg_batch* b) {
     RKDG_CUDA_TRY(cudaEventRecord(b->ev_join, b->stream2));
     RKDG_CUDA_TRY(cudaStreamWaitEvent(b->stream, b->ev_join, 0));
 }
 
-void enqueue_stage(rkdg_batch* b, int s, int in, int u0, int out, bool last) {
+// One stage over the tiles of a chain: order 2 or 1 of two chains, else 0
+// (every tile of the pack in one launch).
+void launch_chain_stage(rkdg_batch* b, const StageArgs& a, int order) {
+    TileArgs t = b->tiles;
+    if (order == 2) t.ntiles = b->n2tiles;
+    if (order == 1) {
+        t.desc = b->tdesc + 2 * (size_t)b->n2tiles;
+        t.ntiles = b->ntiles - b->n2tiles;
+    }
+    if (t.ntiles > 0)
+        launch_stage(a, t, order ? order : b->ord, b->p.nq, b->p.flux, kprec(b), b->ctas,
+                     order == 1 ? b->stream2 : b->stream);
+}
+
+void launch_pack_stage(rkdg_batch* b, const StageArgs& a) {
+    if (!two_chains(b)) return launch_chain_stage(b, a, 0);
+    fork(b);
+    launch_chain_stage(b, a, 2);
+    launch_chain_stage(b, a, 1);
+    join(b);
+}
+
+void enqueue_stage(rkdg_batch* b, int order, int s, int in, int u0, int out, bool last) {
     StageArgs a = stage_args(b);
     coeffs(b->p.rk, s, a.a, a.b);
     a.U = b->U[in];
     a.U0 = s == 0 ? nullptr : b->U[u0];
     a.Unew = b->U[out];
     a.last_stage = last ? 1 : 0;
-    launch_pack_stage(b, a);
+    launch_chain_stage(b, a, order);
 }
 
-void enqueue_step(rkdg_batch* b) {
-    launch_step_begin(b->ctl, b->S, b->stream);
+void enqueue_step(rkdg_batch* b, int order) {
+    launch_step_begin(b->ctl, b->S, order ? order : -1, order == 1 ? b->stream2 : b->stream);
     if (b->p.rk == 3) {
-        enqueue_stage(b, 0, 0, 0, 1, false);
-        enqueue_stage(b, 1, 1, 0, 2, false);
-        enqueue_stage(b, 2, 2, 0, 0, true);
+        enqueue_stage(b, order, 0, 0, 0, 1, false);
+        enqueue_stage(b, order, 1, 1, 0, 2, false);
+        enqueue_stage(b, order, 2, 2, 0, 0, true);
     } else {
-        enqueue_stage(b, 0, 0, 0, 1, false);
-        enqueue_stage(b, 1, 1, 0, 0, true);
+        enqueue_stage(b, order, 0, 0, 0, 1, false);
+        enqueue_stage(b, order, 1, 1, 0, 0, true);
     }
+}
+
+// Whole steps of the pack.  Solves share nothing, so the two chains of a mixed
+// pack run side by side over all the steps and meet only at the end: each
+// fills the SMs that the other's last tiles of a stage leave idle (joined
+// after every stage they waited for each other three times a step).
+void enqueue_steps(rkdg_batch* b, int steps) {
+    const bool two = two_chains(b);
+    if (two) fork(b);
+    for (int i = 0; i < steps; ++i) enqueue_step(b, two ? 2 : 0);
+    if (!two) return;
+    for (int i = 0; i < steps; ++i) enqueue_step(b, 1);
+    join(b);
 }
 
 // (Re)builds the tile tables of every solve for tiles of b->tile elements
@@ -241,7 +269,7 @@ cudaGraphExec_t capture_steps(rkdg_batch* b, int steps) {
     cudaGraph_t g;
     RKDG_CUDA_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     try {
-        for (int i = 0; i < steps; ++i) enqueue_step(b);
+        enqueue_steps(b, steps);
     } catch (...) {
         cudaStreamEndCapture(b->stream, &g);
         throw;
@@ -394,7 +422,10 @@ int rkdg_batch_create(int32_t nsolves, const rkdg_mesh_desc* meshes, const int32
         h2d(b, b->ref32, ref);
         b->staging = (double*)balloc(b, sizeof(double) * 24 * (size_t)maxT);
         b->ctl = (StepCtl*)balloc(b, sizeof(StepCtl) * nsolves);
-        for (int s = 0; s < nsolves; ++s) b->h_ctl[s].cfl = p.cfl;
+        for (int s = 0; s < nsolves; ++s) {
+            b->h_ctl[s].cfl = p.cfl;
+            b->h_ctl[s].chain = orders[s];
+        }
         push(b);
         sync(b);
         *out = b;

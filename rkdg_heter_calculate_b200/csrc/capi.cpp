@@ -212,7 +212,7 @@ void launch_one_stage(rkdg_ctx* c, int s, int in, int u0, int out, bool monitor 
 // one full step on the stream with the state in buffer 0 (graph-capturable);
 // monitor: also form the residual monitor in the last stage
 void enqueue_step(rkdg_ctx* c, bool monitor) {
-    launch_step_begin(c->d.ctl, 1, c->stream);
+    launch_step_begin(c->d.ctl, 1, -1, c->stream);
     if (c->p.rk == 3) {
         launch_one_stage(c, 0, 0, 0, 1, monitor);
         launch_one_stage(c, 1, 1, 0, 2, monitor);
@@ -601,7 +601,7 @@ int rkdg_part_begin_step(rkdg_ctx* c) {
         if (!c->wave_valid) throw Error{RKDG_ERR_STATE, "rkdg_part_begin_step: no wave-speed maximum (rkdg_part_wave)"};
         if (c->pending_stage >= 0) throw Error{RKDG_ERR_STATE, "rkdg_part_begin_step: a stage is still open"};
         RKDG_CUDA_TRY(cudaSetDevice(c->device));
-        launch_step_begin(c->d.ctl, 1, c->stream);
+        launch_step_begin(c->d.ctl, 1, -1, c->stream);
         c->old = c->cur;
         c->wave_valid = false;
     });

@@ -77,11 +77,13 @@ __global__ void reset_wave_kernel(StepCtl* ctl, int n) {
 }
 
 // dt of the step: CFL (or fixed), clipped to land on t_final; advances t.
-__global__ void step_begin_kernel(StepCtl* ctls, int n) {
+__global__ void step_begin_kernel(StepCtl* ctls, int n, int chain) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    grid_dependents_launch();
+    grid_dependency_wait();
     if (i >= n) return;
     StepCtl* ctl = ctls + i;
-    if (ctl->done) return;
+    if (ctl->done || (chain >= 0 && ctl->chain != chain)) return;
     double dt = ctl->dt_fixed > 0 ? ctl->dt_fixed : ctl->cfl / __longlong_as_double((long long)ctl->wave_bits);
     bool last = false;
     if (ctl->t_final > 0) {
@@ -190,6 +192,8 @@ __global__ void __launch_bounds__(kAuxBlock) tiled_limiter_kernel(const TileArgs
                                                               const StepCtl* __restrict__ ctl,
                                                               int* __restrict__ tile_flags,
                                                               int* __restrict__ tile_list, int tile_cap) {
+    grid_dependents_launch();
+    grid_dependency_wait();
     if (tile_list == nullptr) {
         const int ntiles = ta.ntiles_dev ? *ta.ntiles_dev : ta.ntiles;
         for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
@@ -429,6 +433,24 @@ int sm_count() {
 
 namespace {
 
+// Launches a kernel that may start before the one ahead of it in its stream
+// has finished; the kernel calls grid_dependency_wait before it touches
+// anything that one writes.  Only kernels that do so are launched this way.
+template <typename... P, typename... A>
+void launch_dependent(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    RKDG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+
 // Shared-memory attributes of one instantiation for a halo size; returns the
 // dynamic shared memory per CTA.
 
@@ -481,7 +503,7 @@ void launch_tiled(const StageArgs& a, const TileArgs& t, int ctas, cudaStream_t 
     TileArgs ta = t;
     if constexpr (sizeof(Real) == 4)  // FP32 kernels prefetch a device of CTAs ahead (prefetch_ahead)
         if (grid == t.ntiles) ta.ahead = sm_count() * occupancy_tiled<Real, NQ2, FLUX, MODE, ORD, BT>(t.max_halo);
-    if (grid > 0) kernel<<<grid, BT, smem, s>>>(a, ta);
+    if (grid > 0) launch_dependent(kernel, grid, BT, smem, s, a, ta);
 }
 
 // Tile sizes the stage kernel is built for: 128 everywhere, 256 for the
@@ -583,9 +605,8 @@ void launch_wave(const TileArgs& t, int ld, const void* U, int prec, const doubl
     RKDG_CUDA_TRY(cudaGetLastError());
 }
 
-void launch_step_begin(StepCtl* ctl, int nsolves, cudaStream_t stream) {
-    step_begin_kernel<<<(nsolves + 127) / 128, 128, 0, stream>>>(ctl, nsolves);
-    RKDG_CUDA_TRY(cudaGetLastError());
+void launch_step_begin(StepCtl* ctl, int nsolves, int chain, cudaStream_t stream) {
+    launch_dependent(step_begin_kernel, (nsolves + 127) / 128, 128, 0, stream, ctl, nsolves, chain);
 }
 
 namespace {
@@ -645,10 +666,9 @@ void launch_tiled_limiter(const TileArgs& t, int ctas, int ld, void* U, const in
     int grid = ctas > 0 ? ctas : std::max(1, t.ntiles);
     if (tile_list != nullptr && ctas <= 0) grid = std::max(1, std::min(t.ntiles, 4 * sm_count()));
     if (prec == RKDG_FP32)
-        tiled_limiter_kernel<float><<<grid, kAuxBlock, 0, stream>>>(t, ld, static_cast<float*>(U), conn, lim, jinv, flags, refs, gamma, tvb_m, cfg1, cfg2, ctl, tile_flags, tile_list, tile_cap);
+        launch_dependent(tiled_limiter_kernel<float>, grid, kAuxBlock, 0, stream, t, ld, static_cast<float*>(U), conn, lim, jinv, flags, refs, gamma, tvb_m, cfg1, cfg2, ctl, tile_flags, tile_list, tile_cap);
     else
-        tiled_limiter_kernel<double><<<grid, kAuxBlock, 0, stream>>>(t, ld, static_cast<double*>(U), conn, lim, jinv, flags, refs, gamma, tvb_m, cfg1, cfg2, ctl, tile_flags, tile_list, tile_cap);
-    RKDG_CUDA_TRY(cudaGetLastError());
+        launch_dependent(tiled_limiter_kernel<double>, grid, kAuxBlock, 0, stream, t, ld, static_cast<double*>(U), conn, lim, jinv, flags, refs, gamma, tvb_m, cfg1, cfg2, ctl, tile_flags, tile_list, tile_cap);
 }
 
 void launch_rows(bool gather, void* U, int ld, int T, const int* idx, int n, int nrows, void* buf, int* err,

@@ -150,7 +150,7 @@ struct StepCtl {
     int done;
     int error;                 // bit 0: non-physical state seen; bit 1: a device wait timed out;
                                // bit 2: a halo-exchange row index out of range
-    int pad;
+    int chain;                 // which chain of launches advances the solve (launch_step_begin)
 };
 
 // Throws the error a solve's control word reports (no-op when clean).
@@ -289,7 +289,8 @@ void launch_residual(const StageArgs& a, const TileArgs& t, int order, int nq, i
 // state (the far field); `refs` ([solves][4], device) / `ref` (4, host) give it.
 void launch_wave(const TileArgs& t, int ld, const void* U, int prec, const double* jinv,
                  double gamma, StepCtl* ctl, int nsolves, const double* refs, cudaStream_t stream);
-void launch_step_begin(StepCtl* ctl, int nsolves, cudaStream_t stream);
+// dt, time and step count of a step, of the solves of one chain (-1: of all)
+void launch_step_begin(StepCtl* ctl, int nsolves, int chain, cudaStream_t stream);
 // bounded device wait on data that never arrives (see rkdg_wait_selftest)
 void wait_selftest(double limit_s, int* timed_out, double* waited_s);
 // dynamic shared memory per CTA of the tiled stage kernel for a tile size

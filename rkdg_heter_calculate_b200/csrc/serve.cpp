@@ -216,13 +216,11 @@ void coeffs(int rk, int st, double& a, double& c) {
     else a = 1.0 / 3.0, c = 2.0 / 3.0;
 }
 
-// One step of every solve in flight: per RK stage, the stage kernel and the
-// limiter over each tile list (flux, order), the first on the server's
-// stream and the others on streams forked from it (the lists hold different
-// solves, so the launches overlap where one runs out), joined before the
-// next stage.
-void enqueue_step(rkdg_server* s) {
-    launch_step_begin(s->ctl, s->max_slots, s->stream);
+// One step of the solves of one tile list (flux, order): the step's dt, then
+// per RK stage the stage kernel and the limiter.
+void enqueue_step(rkdg_server* s, int l) {
+    const cudaStream_t st_l = l == 0 ? s->stream : s->side[l - 1];
+    launch_step_begin(s->ctl, s->max_slots, l, st_l);
     const int plan[3][3] = {{0, 0, 1}, {1, 0, 2}, {2, 0, 0}};
     const int plan2[2][3] = {{0, 0, 1}, {1, 0, 0}};
     for (int st = 0; st < s->p.rk; ++st) {
@@ -244,22 +242,31 @@ void enqueue_step(rkdg_server* s) {
         a.lo_row = lo_row(s);
         a.tvb_m = s->p.tvb_m;
         a.limiter_on = s->flags;
-        RKDG_CUDA_TRY(cudaEventRecord(s->ev_fork, s->stream));
-        for (int l = 1; l < kLists; ++l) RKDG_CUDA_TRY(cudaStreamWaitEvent(s->side[l - 1], s->ev_fork, 0));
-        for (int l = 0; l < kLists; ++l) {
-            cudaStream_t st_l = l == 0 ? s->stream : s->side[l - 1];
-            a.tile_flags = s->tile_flags + l * s->tcap;
-            a.tile_list = s->tile_list + l * (kListHead + s->tcap);
-            a.tile_cap = (int)s->tcap;
-            launch_stage(a, s->tiles[l], list_order(l), s->p.nq, list_flux(l), kprec(s), s->ctas[l], st_l);
-            launch_tiled_limiter(s->tiles[l], s->ctas[l], s->ld, s->U[pl[2]], s->conn, s->lim, s->jinv, s->flags,
-                                 s->far, kprec(s), s->p.nq, s->p.gamma, s->p.tvb_m, s->ctl, a.tile_flags,
-                                 a.tile_list, a.tile_cap, st_l);
-        }
-        for (int l = 1; l < kLists; ++l) {
-            RKDG_CUDA_TRY(cudaEventRecord(s->ev_join[l - 1], s->side[l - 1]));
-            RKDG_CUDA_TRY(cudaStreamWaitEvent(s->stream, s->ev_join[l - 1], 0));
-        }
+        a.tile_flags = s->tile_flags + l * s->tcap;
+        a.tile_list = s->tile_list + l * (kListHead + s->tcap);
+        a.tile_cap = (int)s->tcap;
+        launch_stage(a, s->tiles[l], list_order(l), s->p.nq, list_flux(l), kprec(s), s->ctas[l], st_l);
+        launch_tiled_limiter(s->tiles[l], s->ctas[l], s->ld, s->U[pl[2]], s->conn, s->lim, s->jinv, s->flags,
+                             s->far, kprec(s), s->p.nq, s->p.gamma, s->p.tvb_m, s->ctl, a.tile_flags,
+                             a.tile_list, a.tile_cap, st_l);
+    }
+}
+
+// Steps per chunk of the loop: one graph launch, one read of the control blocks.
+constexpr int kChunk = 4;
+
+// A chunk of steps of every solve in flight.  The lists hold different solves,
+// which share nothing, so each list's steps are a chain of their own, the first
+// on the server's stream and the others on streams forked from it, and the
+// chains meet at the end of the chunk.
+void enqueue_chunk(rkdg_server* s) {
+    RKDG_CUDA_TRY(cudaEventRecord(s->ev_fork, s->stream));
+    for (int l = 1; l < kLists; ++l) RKDG_CUDA_TRY(cudaStreamWaitEvent(s->side[l - 1], s->ev_fork, 0));
+    for (int l = 0; l < kLists; ++l)
+        for (int i = 0; i < kChunk; ++i) enqueue_step(s, l);
+    for (int l = 1; l < kLists; ++l) {
+        RKDG_CUDA_TRY(cudaEventRecord(s->ev_join[l - 1], s->side[l - 1]));
+        RKDG_CUDA_TRY(cudaStreamWaitEvent(s->stream, s->ev_join[l - 1], 0));
     }
 }
 
@@ -301,6 +308,7 @@ void upload(rkdg_server* s, Request& r) {
                   r.order, kprec(s), r.far, lo_row(s), s->stream);
     StepCtl c{};
     c.cfl = s->p.cfl;
+    c.chain = list_of(r.flux, r.order);
     c.t_final = r.t_final > 0 ? r.t_final : 1e-300;
     h2d(s, s->ctl + r.slot, &c, 1);
     h2d(s, s->far + 4 * r.slot, r.far, 4);
@@ -436,7 +444,6 @@ std::vector<std::shared_ptr<Request>> admit(rkdg_server* s) {
 void engine_loop(rkdg_server* s) {
     try {
         RKDG_CUDA_TRY(cudaSetDevice(s->device));
-        const int chunk = 4;
         while (true) {
             std::vector<std::shared_ptr<Request>> in;
             {
@@ -464,7 +471,7 @@ void engine_loop(rkdg_server* s) {
                 if (s->fault_after > 0) --s->fault_after;
             }
             const double t0 = now_s();
-            for (int i = 0; i < chunk; ++i) RKDG_CUDA_TRY(cudaGraphLaunch(s->graph, s->stream));
+            RKDG_CUDA_TRY(cudaGraphLaunch(s->graph, s->stream));
             RKDG_CUDA_TRY(cudaMemcpyAsync(s->h_ctl, s->ctl, sizeof(StepCtl) * s->max_slots,
                                           cudaMemcpyDeviceToHost, s->stream));
             RKDG_CUDA_TRY(cudaStreamSynchronize(s->stream));
@@ -654,7 +661,7 @@ int rkdg_server_create(const rkdg_params* params, size_t budget, int32_t max_slo
         cudaGraph_t g;
         RKDG_CUDA_TRY(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
         try {
-            enqueue_step(s);
+            enqueue_chunk(s);
         } catch (...) {
             cudaStreamEndCapture(s->stream, &g);
             throw;

@@ -437,9 +437,11 @@ __global__ void __launch_bounds__(BT, Fp64Occupancy<ORD, BT, LAT>::value)
     if (tile >= ntiles) return;
     const int tid = threadIdx.x;
     int4 d0 = __ldg(ta.desc + 2 * tile), d1 = __ldg(ta.desc + 2 * tile + 1);
+    grid_dependents_launch();
     if (tid == 0) mbar_init(&s_bar, 1);
     __syncthreads();
     if (tid == 0) {
+        grid_dependency_wait();
         stage_copy<double, BT>(a, d0, stg, &s_bar);
         stage_prefetch<double, false>(a, ta, d0, d1);
     }
@@ -455,6 +457,7 @@ __global__ void __launch_bounds__(BT, Fp64Occupancy<ORD, BT, LAT>::value)
         // the work that needs only the geometry and the lists, while the state rows arrive
         const int ex = d0.x + (tid < d0.y ? tid : 0);
         const double2 r0 = __ldg(jinv2 + ex), r1 = __ldg(jinv2 + a.ld + ex);
+        grid_dependency_wait();
         const int done = MODE != MODE_RESIDUAL ? a.ctl[d0.z].done : 0;
         if (MODE != MODE_RESIDUAL && tid == 0) s_dt = a.ctl[d0.z].dt;
         if (tid < 4)

@@ -85,6 +85,12 @@ __device__ __forceinline__ uint64_t global_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
+// Programmatic dependent launch (kernels launched by launch_dependent): a
+// kernel lets the next one of its stream start while its own last CTAs run,
+// and the next does what needs only tables (descriptors, geometry, lists) and
+// then waits here until everything before it is complete and visible.
+__device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Waits for the barrier phase of the given parity; gives up after limit_ns
 // nanoseconds (two seconds for the stage kernel's staging waits) or 2^26
 // polls, returning false.
@@ -746,9 +752,13 @@ __global__ void __launch_bounds__(BT, TiledOccupancy<ORD, BT>::value)
     // every thread's descriptor load is in flight while the barrier is set
     // up; nobody waits for the thread that issues the copies
     int4 d0 = __ldg(ta.desc + 2 * tile), d1 = __ldg(ta.desc + 2 * tile + 1);
+    grid_dependents_launch();
     if (threadIdx.x == 0) mbar_init(&s_bar, 1);
     __syncthreads();
-    if (threadIdx.x == 0) stage_copy<Real, BT>(a, d0, stg, &s_bar);
+    if (threadIdx.x == 0) {
+        grid_dependency_wait();
+        stage_copy<Real, BT>(a, d0, stg, &s_bar);
+    }
     __shared__ float2 s_ephi[ORD == 3 ? 2 : 1][3 * kMaxNG * kMaxNB];
     load_edge_table<ORD, NQ2, BT>(g_ephi_f2, s_ephi);  // (read after later barriers)
     const double2* jinv2 = reinterpret_cast<const double2*>(a.jinv);
@@ -760,6 +770,7 @@ __global__ void __launch_bounds__(BT, TiledOccupancy<ORD, BT>::value)
         const int ex = d0.x + ((int)threadIdx.x < d0.y ? (int)threadIdx.x : 0);
         const double2 r0 = __ldg(jinv2 + ex), r1 = __ldg(jinv2 + a.ld + ex);
         const int4 code = __ldg(ta.code + ex);
+        grid_dependency_wait();
         const int done = MODE != MODE_RESIDUAL ? a.ctl[d0.z].done : 0;
         if (MODE != MODE_RESIDUAL && threadIdx.x == 0) s_dt = a.ctl[d0.z].dt;
         const TilePre<Real> pre = tile_pre<Real, BT>(a, ta, d0, d1, r0, r1, code, smem_raw);
