@@ -152,7 +152,7 @@ __device__ __forceinline__ double rk_combine(double u, double u0, double r, doub
 // [2][BT] (LLF); NT threads.
 template <int NG, int FLUX, int BT, int NT>
 __device__ __forceinline__ void flux_tasks64(int nt, const uint16_t* s_task, const int4* s_code, const double* s_nrm,
-                                             double2* s_tr, const double2* s_mean, const double2* s_htr, int HM,
+                                             double2* s_tr, const double2* s_mean, double2* s_htr, int HM,
                                              const double* s_far, double gamma) {
     constexpr int NC = TiledLayout<double, BT>::NC;
     const double gm1 = add_(gamma, -1.0);
@@ -167,7 +167,8 @@ __device__ __forceinline__ void flux_tasks64(int nt, const uint16_t* s_task, con
         roots_f64(fma(Nx, Nx, mul_(Ny, Ny)), len, il);
         const double nx = mul_(Nx, il), ny = mul_(Ny, il);
         // the other side's values: in-tile slots, or the halo rows
-        const double2* nb = kind == EDGE_HALO ? s_htr + idx : s_tr + (size_t)2 * se * NG * BT + idx;
+        const bool bnd = kind == EDGE_BOUNDARY;
+        double2* nb = kind == EDGE_HALO ? s_htr + idx : s_tr + 2 * se * NG * BT + idx;
         const int nld = kind == EDGE_HALO ? HM : BT;
         double alpha = 0.0;
         if constexpr (FLUX == RKDG_FLUX_LLF) {
@@ -191,13 +192,11 @@ __device__ __forceinline__ void flux_tasks64(int nt, const uint16_t* s_task, con
             double uR[4], f[4];
             // the neighbour's point NG-1-g on its edge se pairs with ours
             // (src/kernelfunctions.cu:545-549)
-            const double2* np = nb + 2 * (NG - 1 - g) * nld;
-            if (kind == EDGE_BOUNDARY) {
-                ghost<double>(se, uL, s_far, nx, ny, uR);
-            } else {
-                x = np[0], y = np[nld];
-                uR[0] = x.x, uR[1] = x.y, uR[2] = y.x, uR[3] = y.y;
-            }
+            // of a boundary edge the other slot is the own one
+            double2* np = bnd ? slot : nb + 2 * (NG - 1 - g) * nld;
+            x = np[0], y = np[nld];
+            uR[0] = x.x, uR[1] = x.y, uR[2] = y.x, uR[3] = y.y;
+            if (bnd) ghost<double>(se, uL, s_far, nx, ny, uR);
             if constexpr (FLUX == RKDG_FLUX_LLF) {
                 llf_flux(uL, uR, Nx, Ny, alpha, gm1, f);
             } else {
@@ -205,15 +204,14 @@ __device__ __forceinline__ void flux_tasks64(int nt, const uint16_t* s_task, con
 #pragma unroll
                 for (int v = 0; v < 4; ++v) f[v] = mul_(f[v], len);
             }
-            // each slot of an edge is read by this task alone: the computing
-            // side's slot takes the flux, an in-tile neighbour's its negation
+            // each slot of an edge is read by this task alone: the other
+            // side's slot takes the negated flux (an in-tile neighbour's; a
+            // halo's is read no more; a boundary's is overwritten at once),
+            // the computing side's the flux
+            np[0] = make_double2(-f[0], -f[1]);
+            np[nld] = make_double2(-f[2], -f[3]);
             slot[0] = make_double2(f[0], f[1]);
             slot[BT] = make_double2(f[2], f[3]);
-            if (kind == EDGE_IN_OWNER) {
-                double2* ns = const_cast<double2*>(np);
-                ns[0] = make_double2(-f[0], -f[1]);
-                ns[BT] = make_double2(-f[2], -f[3]);
-            }
         }
     }
 }

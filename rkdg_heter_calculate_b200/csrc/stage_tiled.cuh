@@ -386,6 +386,10 @@ __device__ __forceinline__ void flux_tasks32(int nt, const uint16_t* s_task, con
         Real len, il;
         lengths_(fma(Nx, Nx, mul_(Ny, Ny)), len, il);
         const Real nx = mul_(Nx, il), ny = mul_(Ny, il);
+        const bool bnd = kind == EDGE_BOUNDARY;
+        // the other side's slots: halo rows or in-tile slots
+        V4* other = kind == EDGE_HALO ? s_htr + idx : s_tr + se * NG * BT + idx;
+        const int stride = kind == EDGE_HALO ? HM : BT;
         Real alpha = Real(0);
         if constexpr (MEANS) {
             Real mL[4], mR[4];
@@ -400,10 +404,11 @@ __device__ __forceinline__ void flux_tasks32(int nt, const uint16_t* s_task, con
             V4* slot = s_tr + (k * NG + g) * BT + le;
             get4(slot, uL);
             // the neighbour's point NG-1-g on its edge se pairs with ours
-            // (src/kernelfunctions.cu:545-549)
-            V4* nslot = kind == EDGE_HALO ? s_htr + (NG - 1 - g) * HM + idx : s_tr + (se * NG + NG - 1 - g) * BT + idx;
-            if (kind == EDGE_BOUNDARY) ghost_dev<Real>(se, uL, rs, nx, ny, uR);
-            else get4(nslot, uR);
+            // (src/kernelfunctions.cu:545-549); of a boundary edge the other
+            // slot is the own one
+            V4* nslot = bnd ? slot : other + (NG - 1 - g) * stride;
+            get4(nslot, uR);
+            if (bnd) ghost_dev<Real>(se, uL, rs, nx, ny, uR);
             Real fh[4], fn[4];  // the flux out of this side and into the neighbour
             if (FLUX == RKDG_FLUX_LLF) {
                 Real fL[4], fR[4];
@@ -422,10 +427,12 @@ __device__ __forceinline__ void flux_tasks32(int nt, const uint16_t* s_task, con
                 set4(fh, f2mul(lo2(f), l), f2mul(hi2(f), l));
                 set4(fn, f2mul(lo2(f), nl), f2mul(hi2(f), nl));
             }
-            // each slot of an edge is read by this task alone: the computing
-            // side's slot takes the flux, an in-tile neighbour's its negation
+            // each slot of an edge is read by this task alone: the other
+            // side's slot takes the negated flux (an in-tile neighbour's; a
+            // halo's is read no more; a boundary's is overwritten at once),
+            // the computing side's the flux
+            put4(nslot, fn);
             put4(slot, fh);
-            if (kind == EDGE_IN_OWNER) put4(nslot, fn);
         }
     }
 }
