@@ -43,6 +43,7 @@ struct rkdg_ctx {
     cudaGraphExec_t graph = nullptr;    // one step
     cudaGraphExec_t graph_n = nullptr;  // kGraphSteps steps (fewer graph launches and boundaries)
     StepCtl* h_ctl = nullptr;  // pinned mirror of the device control block
+    bool ctl_fresh = false;    // the mirror equals the device's (nothing that writes it enqueued since the last pull)
     TileArgs tiles{};
     int ctas = 0;     // tiled grid size (0: one CTA per tile)
     int n_int_tiles = 0;     // a partition's tiles that read no halo copy (they come first)
@@ -132,6 +133,7 @@ void ensure_conversion(rkdg_ctx* c) {
 void pull_ctl(rkdg_ctx* c) {
     RKDG_CUDA_TRY(cudaMemcpyAsync(c->h_ctl, c->d.ctl, sizeof(StepCtl), cudaMemcpyDeviceToHost, c->stream));
     sync(c);
+    c->ctl_fresh = true;
 }
 
 void push_ctl(rkdg_ctx* c) {
@@ -154,6 +156,7 @@ void normalise_buffers(rkdg_ctx* c) {
 
 void ensure_wave(rkdg_ctx* c) {
     if (c->wave_valid) return;
+    c->ctl_fresh = false;
     launch_wave(c->tiles, c->ld, c->d.U[c->cur], kprec(c), c->d.jinv, c->p.gamma, c->d.ctl, 1,
                 c->d.far, c->stream);
     c->wave_valid = true;
@@ -187,6 +190,7 @@ void stage_coeffs(int rk, int s, double& a, double& b) {
 }
 
 void launch_one_stage(rkdg_ctx* c, int s, int in, int u0, int out, bool monitor = true, bool part_stage = false) {
+    c->ctl_fresh = false;
     StageArgs a = base_args(c);
     stage_coeffs(c->p.rk, s, a.a, a.b);
     a.U = c->d.U[in];
@@ -226,6 +230,7 @@ void enqueue_step(rkdg_ctx* c, bool monitor) {
 // `steps` whole steps (at most kResidentSteps) in one launch, with the state
 // in buffer 0
 void enqueue_resident(rkdg_ctx* c, int steps, bool monitor) {
+    c->ctl_fresh = false;
     StageArgs a = base_args(c);
     a.Unew = c->d.U[0];
     a.far_sid = c->d.far;
@@ -254,6 +259,7 @@ cudaGraphExec_t capture_steps(rkdg_ctx* c, int steps, bool monitor) {
 }
 
 void check_error_flag(rkdg_ctx* c) {
+    if (c->h_ctl->error) c->rw.clean = false;
     throw_ctl_error(c->h_ctl->error, "solve");
 }
 
@@ -271,6 +277,7 @@ int stage_output(const rkdg_ctx* c, int s) {
 // the caller (rkdg_part_limit), as in rkdg_part_stage.
 void launch_part_tiles(rkdg_ctx* c, int s, int out, int first, int last) {
     if (last <= first) return;
+    c->ctl_fresh = false;
     StageArgs a = base_args(c);
     stage_coeffs(c->p.rk, s, a.a, a.b);
     a.U = c->d.U[c->cur];
@@ -549,6 +556,7 @@ int rkdg_gather_rows(rkdg_ctx* c, const int32_t* d_index, int32_t n, int32_t nro
             throw Error{RKDG_ERR_INVALID, "rkdg_gather_rows: bad arguments"};
         require_state(c);
         RKDG_CUDA_TRY(cudaSetDevice(c->device));
+        c->ctl_fresh = false;
         launch_rows(true, c->d.U[c->cur], c->ld, c->T, d_index, n, nrows, d_out, &c->d.ctl->error, c->stream);
     });
 }
@@ -559,6 +567,7 @@ int rkdg_scatter_rows(rkdg_ctx* c, const int32_t* d_index, int32_t n, int32_t nr
             throw Error{RKDG_ERR_INVALID, "rkdg_scatter_rows: bad arguments"};
         require_state(c);
         RKDG_CUDA_TRY(cudaSetDevice(c->device));
+        c->ctl_fresh = false;
         launch_rows(false, c->d.U[c->cur], c->ld, c->T, d_index, n, nrows, const_cast<void*>(d_in),
                     &c->d.ctl->error, c->stream);
     });
@@ -585,6 +594,7 @@ int rkdg_part_wave(rkdg_ctx* c, double* d_wave, int32_t to_context) {
         // the maximum is kept as the bits of a non-negative double
         unsigned long long* w = &c->d.ctl->wave_bits;
         if (to_context) {
+            c->ctl_fresh = false;
             RKDG_CUDA_TRY(cudaMemcpyAsync(w, d_wave, sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
             c->wave_valid = true;
         } else {
@@ -601,6 +611,7 @@ int rkdg_part_begin_step(rkdg_ctx* c) {
         if (!c->wave_valid) throw Error{RKDG_ERR_STATE, "rkdg_part_begin_step: no wave-speed maximum (rkdg_part_wave)"};
         if (c->pending_stage >= 0) throw Error{RKDG_ERR_STATE, "rkdg_part_begin_step: a stage is still open"};
         RKDG_CUDA_TRY(cudaSetDevice(c->device));
+        c->ctl_fresh = false;
         launch_step_begin(c->d.ctl, 1, -1, c->stream);
         c->old = c->cur;
         c->wave_valid = false;
@@ -760,6 +771,7 @@ int rkdg_residual(rkdg_ctx* c, double* R, int32_t ld, int32_t basis) {
         ensure_staging(c);
         if (basis == RKDG_BASIS_REFERENCE) ensure_conversion(c);
         else if (basis != RKDG_BASIS_NATIVE) throw Error{RKDG_ERR_INVALID, "unknown basis"};
+        c->ctl_fresh = false;
         // scratch: a buffer that holds neither the current nor the saved state
         int scratch = 0;
         while (scratch == c->cur || scratch == c->old) ++scratch;
@@ -845,11 +857,17 @@ int rkdg_step(rkdg_ctx* c, double dt, double* dt_used, double* monitor) {
         RKDG_CUDA_TRY(cudaSetDevice(c->device));
         normalise_buffers(c);
         ensure_wave(c);
-        pull_ctl(c);
-        c->h_ctl->dt_fixed = dt > 0 ? dt : 0.0;
-        c->h_ctl->t_final = 0.0;
-        c->h_ctl->done = 0;
-        push_ctl(c);
+        // the previous step's read-back usually still holds: a host loop then
+        // pays one launch and one read-back per step
+        if (!c->ctl_fresh) pull_ctl(c);
+        const double fixed = dt > 0 ? dt : 0.0;
+        if (c->h_ctl->dt_fixed != fixed || c->h_ctl->t_final != 0.0 || c->h_ctl->done != 0) {
+            c->h_ctl->dt_fixed = fixed;
+            c->h_ctl->t_final = 0.0;
+            c->h_ctl->done = 0;
+            push_ctl(c);
+        }
+        c->ctl_fresh = false;
         if (c->resident) enqueue_resident(c, 1, true);
         else enqueue_step(c, true);
         c->wave_valid = true;
@@ -879,6 +897,7 @@ int rkdg_advance(rkdg_ctx* c, int32_t nsteps, double t_final, double* t, int32_t
         c->h_ctl->t_final = t_final > 0 ? t_final : 0.0;
         c->h_ctl->done = 0;
         push_ctl(c);
+        c->ctl_fresh = false;
         if (c->resident) {
             int left = nsteps;
             while (left > 0) {
@@ -916,7 +935,7 @@ int rkdg_advance(rkdg_ctx* c, int32_t nsteps, double t_final, double* t, int32_t
             for (int i = 0; i < nsteps; ++i) {
                 const int before = c->h_ctl->step;
                 RKDG_CUDA_TRY(cudaGraphLaunch(c->graph, c->stream));
-                pull_ctl(c);
+                pull_ctl(c);  // (the last one leaves the mirror current)
                 if (c->h_ctl->step == before || c->h_ctl->error) break;  // done or failed
                 log_residual(c);
             }
@@ -928,6 +947,7 @@ int rkdg_advance(rkdg_ctx* c, int32_t nsteps, double t_final, double* t, int32_t
         const int chunk = t_final > 0 ? 64 : nsteps;
         while (left > 0) {
             int n = std::min(left, chunk > 0 ? chunk : 1);
+            c->ctl_fresh = false;
             for (int i = 0; i < n / kGraphSteps && c->graph_n; ++i)
                 RKDG_CUDA_TRY(cudaGraphLaunch(c->graph_n, c->stream));
             for (int i = c->graph_n ? n / kGraphSteps * kGraphSteps : 0; i < n; ++i)
@@ -957,6 +977,7 @@ int rkdg_time_stage(rkdg_ctx* c, int32_t s, int32_t reps, double* ms) {
         if (!(c->h_ctl->dt > 0)) c->h_ctl->dt = 1e-6;
         c->h_ctl->done = 0;
         push_ctl(c);
+        c->ctl_fresh = false;
         // input buffer 0 (the state), U^n = buffer 0, output buffer 1: a
         // stage that writes neither its input nor U^n, so launches repeat
         StageArgs a = base_args(c);

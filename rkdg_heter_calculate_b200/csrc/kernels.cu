@@ -434,10 +434,10 @@ int sm_count() {
 namespace {
 
 // Launches a kernel that may start before the one ahead of it in its stream
-// has finished; the kernel calls grid_dependency_wait before it touches
+// has finished (early); the kernel calls grid_dependency_wait before it touches
 // anything that one writes.  Only kernels that do so are launched this way.
 template <typename... P, typename... A>
-void launch_dependent(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
+void launch_dependent(bool early, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
@@ -447,7 +447,7 @@ void launch_dependent(void (*kernel)(P...), int grid, int block, size_t smem, cu
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early ? 1 : 0;
     RKDG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
 }
 
@@ -501,9 +501,19 @@ void launch_tiled(const StageArgs& a, const TileArgs& t, int ctas, cudaStream_t 
     const int grid = (ctas > 0 && ctas < t.ntiles) ? ctas : t.ntiles;
     constexpr auto kernel = stage_kernel<Real, NQ2, FLUX, MODE, ORD, BT, LAT>();
     TileArgs ta = t;
-    if constexpr (sizeof(Real) == 4)  // FP32 kernels prefetch a device of CTAs ahead (prefetch_ahead)
-        if (grid == t.ntiles) ta.ahead = sm_count() * occupancy_tiled<Real, NQ2, FLUX, MODE, ORD, BT>(t.max_halo);
-    if (grid > 0) launch_dependent(kernel, grid, BT, smem, s, a, ta);
+    // FP32 kernels prefetch a device of CTAs ahead (prefetch_ahead).  Below 7/8
+    // of such a device they start only after the launch before: CTAs that start
+    // early fill the free places of some SMs, and a stage of less than one wave
+    // then runs unevenly spread (FP32C P2, 565 tiles of 888: 38.8 us a step
+    // against 32.3; from 792 tiles on 40.3 against 41.6).  FP64 gains at every
+    // size (352 to 3,907 tiles: 1-4 %).
+    bool early = true;
+    if constexpr (sizeof(Real) == 4) {
+        const int device = sm_count() * occupancy_tiled<Real, NQ2, FLUX, MODE, ORD, BT>(t.max_halo);
+        if (grid == t.ntiles) ta.ahead = device;
+        early = 8 * (int64_t)grid >= 7 * (int64_t)device;
+    }
+    if (grid > 0) launch_dependent(early, kernel, grid, BT, smem, s, a, ta);
 }
 
 // Tile sizes the stage kernel is built for: 128 everywhere, 256 for the
@@ -606,7 +616,7 @@ void launch_wave(const TileArgs& t, int ld, const void* U, int prec, const doubl
 }
 
 void launch_step_begin(StepCtl* ctl, int nsolves, int chain, cudaStream_t stream) {
-    launch_dependent(step_begin_kernel, (nsolves + 127) / 128, 128, 0, stream, ctl, nsolves, chain);
+    launch_dependent(true, step_begin_kernel, (nsolves + 127) / 128, 128, 0, stream, ctl, nsolves, chain);
 }
 
 namespace {
@@ -666,9 +676,9 @@ void launch_tiled_limiter(const TileArgs& t, int ctas, int ld, void* U, const in
     int grid = ctas > 0 ? ctas : std::max(1, t.ntiles);
     if (tile_list != nullptr && ctas <= 0) grid = std::max(1, std::min(t.ntiles, 4 * sm_count()));
     if (prec == RKDG_FP32)
-        launch_dependent(tiled_limiter_kernel<float>, grid, kAuxBlock, 0, stream, t, ld, static_cast<float*>(U), conn, lim, jinv, flags, refs, gamma, tvb_m, cfg1, cfg2, ctl, tile_flags, tile_list, tile_cap);
+        launch_dependent(true, tiled_limiter_kernel<float>, grid, kAuxBlock, 0, stream, t, ld, static_cast<float*>(U), conn, lim, jinv, flags, refs, gamma, tvb_m, cfg1, cfg2, ctl, tile_flags, tile_list, tile_cap);
     else
-        launch_dependent(tiled_limiter_kernel<double>, grid, kAuxBlock, 0, stream, t, ld, static_cast<double*>(U), conn, lim, jinv, flags, refs, gamma, tvb_m, cfg1, cfg2, ctl, tile_flags, tile_list, tile_cap);
+        launch_dependent(true, tiled_limiter_kernel<double>, grid, kAuxBlock, 0, stream, t, ld, static_cast<double*>(U), conn, lim, jinv, flags, refs, gamma, tvb_m, cfg1, cfg2, ctl, tile_flags, tile_list, tile_cap);
 }
 
 void launch_rows(bool gather, void* U, int ld, int T, const int* idx, int n, int nrows, void* buf, int* err,

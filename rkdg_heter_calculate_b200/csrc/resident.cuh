@@ -47,9 +47,9 @@ struct ResidentArgs {
     ulonglong2* trace;   // [2][rows][2][slots] the exchanged traces and means (LLF)
     ulonglong2* mean;    // [2][mean rows][2][slots] the exchanged means of a limited stage
     unsigned epoch;      // stages numbered before this launch
-    unsigned long long* wave;  // [nsteps] zeroed: per-step wave-speed maxima, as bits
-    unsigned* count;           // [nsteps] zeroed: tiles that have added theirs
-    unsigned long long* mon;   // [2] zeroed: the monitor of a one-step launch
+    unsigned long long* wave;  // [nsteps] zero before and after: per-step wave-speed maxima, as bits
+    unsigned* count;           // [nsteps] likewise: tiles that have added theirs
+    unsigned long long* mon;   // [2] likewise: the monitor of a one-step launch
 };
 
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
@@ -229,6 +229,7 @@ __global__ void __launch_bounds__(NT, (sizeof(Real) == 8 ? 256 : 512) / NT) resi
     if (tid == CT) {
         if (t_final > 0 && !(t_final - t > 0)) done = 1;
         s_end = done;
+        s_stop = 0;
     }
     unsigned ep = a.epoch;
     bool ok = true;
@@ -551,6 +552,12 @@ finished:
         if (bad_dt) atomicOr(&c->error, 1);
     }
     if (__syncthreads_or(!ok)) goto lost;
+    // every tile has counted itself into the last step, so none will read the
+    // sums again: zero for the next launch (after an error the host clears them)
+    if (blockIdx.x == 0 && !s_stop) {
+        for (int i = tid; i < a.nsteps; i += NT) a.wave[i] = 0ull, a.count[i] = 0u;
+        if (tid < 2) a.mon[tid] = 0ull;
+    }
     return;
 lost:  // a wait ran out: report and leave (the other tiles' waits run out too)
     if (tid == 0) atomicOr(&a.ctl->error, 2);
@@ -636,7 +643,8 @@ void launch_resident_of(const StageArgs& a, const TileArgs& t, const void* lim, 
     r.mon = r.wave + kResidentSteps;
     r.count = reinterpret_cast<unsigned*>(r.mon + 2);
     w.epoch += (unsigned)(steps * rk);
-    RKDG_CUDA_TRY(cudaMemsetAsync(w.sums, 0, kResidentSums, stream));
+    if (!w.clean) RKDG_CUDA_TRY(cudaMemsetAsync(w.sums, 0, kResidentSums, stream));
+    w.clean = true;  // each launch leaves them so, unless it reports an error
     with_resident<Real>(order, nq, flux, lim != nullptr, a.lo_row >= 0, [&](auto form) { form.launch(r, t, stream); });
 }
 

@@ -258,6 +258,7 @@ struct ResidentWork {            // a context's exchange buffers
     void* trace = nullptr;       // [2][rows][2][slots] 16 bytes, zero before the first launch
     void* mean = nullptr;        // with the limiter, likewise
     unsigned char* sums = nullptr;  // per-step maxima and counts of one launch, the monitor
+    bool clean = false;          // sums are zero for the next launch
     unsigned epoch = 0;          // stages numbered so far
 };
 constexpr int kResidentSteps = 64;  // most steps of one launch
