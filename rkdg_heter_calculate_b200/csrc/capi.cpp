@@ -228,14 +228,16 @@ void enqueue_step(rkdg_ctx* c, bool monitor) {
 }
 
 // `steps` whole steps (at most kResidentSteps) in one launch, with the state
-// in buffer 0
-void enqueue_resident(rkdg_ctx* c, int steps, bool monitor) {
+// in buffer 0; false: the device does not take the launch, and the context
+// uses the stage kernels from here on
+bool enqueue_resident(rkdg_ctx* c, int steps, bool monitor) {
     c->ctl_fresh = false;
     StageArgs a = base_args(c);
     a.Unew = c->d.U[0];
     a.far_sid = c->d.far;
-    launch_resident(a, c->tiles, c->p.limiter == RKDG_LIMITER_TVB ? c->d.lim : nullptr, c->rw, c->p.order, c->p.nq,
-                    c->p.flux, kprec(c), c->p.rk, steps, monitor, c->stream);
+    c->resident = launch_resident(a, c->tiles, c->p.limiter == RKDG_LIMITER_TVB ? c->d.lim : nullptr, c->rw,
+                                  c->p.order, c->p.nq, c->p.flux, kprec(c), c->p.rk, steps, monitor, c->stream);
+    return c->resident;
 }
 
 constexpr int kGraphSteps = 8;
@@ -868,8 +870,7 @@ int rkdg_step(rkdg_ctx* c, double dt, double* dt_used, double* monitor) {
             push_ctl(c);
         }
         c->ctl_fresh = false;
-        if (c->resident) enqueue_resident(c, 1, true);
-        else enqueue_step(c, true);
+        if (!c->resident || !enqueue_resident(c, 1, true)) enqueue_step(c, true);
         c->wave_valid = true;
         pull_ctl(c);
         check_error_flag(c);
@@ -903,7 +904,7 @@ int rkdg_advance(rkdg_ctx* c, int32_t nsteps, double t_final, double* t, int32_t
             while (left > 0) {
                 const int n = c->reslog ? 1 : std::min(left, kResidentSteps);
                 const int before = c->h_ctl->step;
-                enqueue_resident(c, n, (bool)c->reslog);
+                if (!enqueue_resident(c, n, (bool)c->reslog)) break;
                 left -= n;
                 // with a final time, stop once the device says done; the
                 // history needs every step's monitor
@@ -915,6 +916,9 @@ int rkdg_advance(rkdg_ctx* c, int32_t nsteps, double t_final, double* t, int32_t
                 }
             }
             if (c->reslog) c->reslog->flush();
+            nsteps = left;  // (a refused launch: the rest below)
+        }
+        if (c->resident) {
             c->wave_valid = true;
             pull_ctl(c);
             check_error_flag(c);

@@ -584,9 +584,9 @@ int resident_tiles(int prec, int order, int nq, int flux, bool limiter, bool com
     return (prec == RKDG_FP32 ? resident_tiles_fp32 : resident_tiles_fp64)(order, nq, flux, limiter, comp, max_halo);
 }
 
-void launch_resident(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
+bool launch_resident(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
                      int flux, int prec, int rk, int steps, bool monitor, cudaStream_t stream) {
-    (prec == RKDG_FP32 ? launch_resident_fp32 : launch_resident_fp64)(a, t, lim, w, order, nq, flux, rk, steps, monitor,
+    return (prec == RKDG_FP32 ? launch_resident_fp32 : launch_resident_fp64)(a, t, lim, w, order, nq, flux, rk, steps, monitor,
                                                                       stream);
 }
 

@@ -591,12 +591,19 @@ struct ResidentForm {
     }
     static int tiles(int max_halo) { return std::max(fit<256>(max_halo), fit<128>(max_halo)); }
     // 256 threads per tile while the device holds all tiles that way
-    static void launch(ResidentArgs a, TileArgs t, cudaStream_t s) {
+    // (false: refused as a whole, as under a limit on the SMs a process may use)
+    static bool launch(ResidentArgs a, TileArgs t, cudaStream_t s) {
         void* args[] = {&a, &t};
         const bool wide = t.ntiles <= fit<256>(t.max_halo);
         const void* k = wide ? (const void*)kernel<256>() : (const void*)kernel<128>();
-        RKDG_CUDA_TRY(cudaLaunchCooperativeKernel(k, dim3(t.ntiles), dim3(wide ? 256 : 128), args,
-                                                  SM::bytes(t.max_halo), s));
+        const cudaError_t e = cudaLaunchCooperativeKernel(k, dim3(t.ntiles), dim3(wide ? 256 : 128), args,
+                                                          SM::bytes(t.max_halo), s);
+        if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+            cudaGetLastError();
+            return false;
+        }
+        RKDG_CUDA_TRY(e);
+        return true;
     }
 };
 
@@ -630,7 +637,7 @@ auto with_resident(int order, int nq, int flux, bool limiter, bool comp, F&& f) 
 }
 
 template <typename Real>
-void launch_resident_of(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
+bool launch_resident_of(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
                         int flux, int rk, int steps, bool monitor, cudaStream_t stream) {
     ResidentArgs r{};
     r.U = a.Unew;
@@ -645,7 +652,8 @@ void launch_resident_of(const StageArgs& a, const TileArgs& t, const void* lim, 
     w.epoch += (unsigned)(steps * rk);
     if (!w.clean) RKDG_CUDA_TRY(cudaMemsetAsync(w.sums, 0, kResidentSums, stream));
     w.clean = true;  // each launch leaves them so, unless it reports an error
-    with_resident<Real>(order, nq, flux, lim != nullptr, a.lo_row >= 0, [&](auto form) { form.launch(r, t, stream); });
+    return with_resident<Real>(order, nq, flux, lim != nullptr, a.lo_row >= 0,
+                               [&](auto form) { return form.launch(r, t, stream); });
 }
 
 }  // namespace

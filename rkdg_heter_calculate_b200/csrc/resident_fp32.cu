@@ -9,9 +9,9 @@ int resident_tiles_fp32(int order, int nq, int flux, bool limiter, bool comp, in
     return with_resident<float>(order, nq, flux, limiter, comp, [&](auto form) { return form.tiles(max_halo); });
 }
 
-void launch_resident_fp32(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
+bool launch_resident_fp32(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
                           int flux, int rk, int steps, bool monitor, cudaStream_t stream) {
-    launch_resident_of<float>(a, t, lim, w, order, nq, flux, rk, steps, monitor, stream);
+    return launch_resident_of<float>(a, t, lim, w, order, nq, flux, rk, steps, monitor, stream);
 }
 
 void upload_resident_tables_fp32(int nq, int ng) { upload_module_tables(nq, ng); }

@@ -9,9 +9,9 @@ int resident_tiles_fp64(int order, int nq, int flux, bool limiter, bool comp, in
     return with_resident<double>(order, nq, flux, limiter, comp, [&](auto form) { return form.tiles(max_halo); });
 }
 
-void launch_resident_fp64(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
+bool launch_resident_fp64(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
                           int flux, int rk, int steps, bool monitor, cudaStream_t stream) {
-    launch_resident_of<double>(a, t, lim, w, order, nq, flux, rk, steps, monitor, stream);
+    return launch_resident_of<double>(a, t, lim, w, order, nq, flux, rk, steps, monitor, stream);
 }
 
 void upload_resident_tables_fp64(int nq, int ng) { upload_module_tables(nq, ng); }

@@ -267,13 +267,14 @@ int resident_tiles(int prec, int order, int nq, int flux, bool limiter, bool com
 // its tables (each CUDA translation unit holds its own)
 void upload_resident_tables_fp32(int nq, int ng);
 void upload_resident_tables_fp64(int nq, int ng);
-void launch_resident(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
+// (false: the device refused to hold the launch as a whole; nothing was enqueued but the sums' clearing)
+bool launch_resident(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
                      int flux, int prec, int rk, int steps, bool monitor, cudaStream_t stream);
 int resident_tiles_fp32(int order, int nq, int flux, bool limiter, bool comp, int max_halo);
 int resident_tiles_fp64(int order, int nq, int flux, bool limiter, bool comp, int max_halo);
-void launch_resident_fp32(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
+bool launch_resident_fp32(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
                           int flux, int rk, int steps, bool monitor, cudaStream_t stream);
-void launch_resident_fp64(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
+bool launch_resident_fp64(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
                           int flux, int rk, int steps, bool monitor, cudaStream_t stream);
 // The tile-staged stage kernel: one CTA per tile of kTile elements (each
 // interior flux once per tile, traces shared in shared memory), `ctas` CTAs

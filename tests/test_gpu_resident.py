@@ -100,3 +100,32 @@ def test_resident_reports_a_non_physical_state():
         s.advance(5)
     assert e.value.code == 4
     s.close()
+
+
+def test_resident_solves_in_several_threads():
+    """Launches that each fill the device, from contexts in several host
+    threads: each gets the device as a whole, one after the other, and gives
+    the bits it gives alone."""
+    import threading
+
+    kw = dict(order=2, nq=6, ng=3, flux="hllc", precision="fp64", cfl=0.2, farfield=FAR)
+    mesh = meshgen.periodic_structured(136, 136, jitter=0.15, seed=3)
+    U = start(mesh, 6, FAR, "vortex")
+
+    def solve(out, i):
+        s = CUDARkdgSolver(mesh, **kw)
+        s.setFreedom(U, basis="native")
+        for _ in range(4):
+            s.advance(70)
+        out[i] = s.copyFreedomToHost(basis="native")
+        s.close()
+
+    alone, together = [None], [None] * 4
+    solve(alone, 0)
+    threads = [threading.Thread(target=solve, args=(together, i)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for out in together:
+        np.testing.assert_array_equal(out, alone[0])
