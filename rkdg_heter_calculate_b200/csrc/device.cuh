@@ -544,13 +544,13 @@ __device__ __forceinline__ void tvb_geometry(Real c0x, Real c0y, Real c1x, Real 
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const Real dxi = k == 1 ? Real(-1.0 / 3.0) : Real(1.0 / 6.0), deta = k == 2 ? Real(-1.0 / 3.0) : Real(1.0 / 6.0);
-        const Real dx = c0x * dxi + c1x * deta, dy = c0y * dxi + c1y * deta;
-        const Real r2 = dx * dx + dy * dy;
+        const Real dx = fma(c0x, dxi, mul_(c1x, deta)), dy = fma(c0y, dxi, mul_(c1y, deta));
+        const Real r2 = fma(dx, dx, mul_(dy, dy));
         Real rl, irl;
         lengths_(r2, rl, irl);
-        dirx[k] = dx * irl;
-        diry[k] = dy * irl;
-        thr[k] = tvb_m * (Real(4) * r2);
+        dirx[k] = mul_(dx, irl);
+        diry[k] = mul_(dy, irl);
+        thr[k] = mul_(tvb_m, mul_(Real(4), r2));
     }
 }
 #include "stage_tiled.cuh"
@@ -570,10 +570,10 @@ template <typename Real>
 using LimitPair = typename std::conditional<sizeof(Real) == 8, double2, float2>::type;
 // The new P1 modes m1, m2 of an element from its mean, its modes and the
 // neighbours' means near (filled in here across boundary edges); false when
-// every characteristic increment is kept.  Not inlined: every kernel that
-// limits runs this one function, so all limit to the same bits.
+// every characteristic increment is kept.  Sums of products are spelled out
+// (add_, mul_, fma), so every kernel that limits gives the same bits.
 template <typename Real>
-__device__ __noinline__ bool limit_modes(double2 r0, double2 r1, int4 cn, const LimitPair<Real> ab[3],
+__device__ __forceinline__ bool limit_modes(double2 r0, double2 r1, int4 cn, const LimitPair<Real> ab[3],
                                          const Real mean[4], Real near[3][4], Real m1[4], Real m2[4], Real gamma,
                                          Real tvb_m, const double* farp, const Tab<Real>* tbp) {
     const Tab<Real>& tb = *tbp;
@@ -581,41 +581,41 @@ __device__ __noinline__ bool limit_modes(double2 r0, double2 r1, int4 cn, const 
     const unsigned pair_bits = ((unsigned)cn.w >> 12) & 7u;
     // the directions and threshold scales in the working precision: FP64
     // for the parity path, FP32 (from the FP64 J^-1 rows) for the FP32 forms
-    const Real idet = rcp_((Real)(r0.x * r1.y - r0.y * r1.x));  // det J
+    const Real idet = rcp_((Real)fma(r0.x, r1.y, -mul_(r0.y, r1.x)));  // det J
     // columns of J: x_1 - x_0 and x_2 - x_0
     Real dirx[3], diry[3], thrk[3];
-    tvb_geometry<Real>((Real)r1.y * idet, -(Real)r1.x * idet, -(Real)r0.y * idet, (Real)r0.x * idet, tvb_m, dirx,
-                       diry, thrk);
+    tvb_geometry<Real>(mul_((Real)r1.y, idet), -mul_((Real)r1.x, idet), -mul_((Real)r0.y, idet), mul_((Real)r0.x, idet),
+                       tvb_m, dirx, diry, thrk);
     Real tmax = Real(0);
 #pragma unroll
     for (int k = 0; k < 3; ++k)
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
-            tilde[k][v] = tb.mphi[k][0] * m1[v] + tb.mphi[k][1] * m2[v];
+            tilde[k][v] = fma(tb.mphi[k][0], m1[v], mul_(tb.mphi[k][1], m2[v]));
             tmax = fmax(tmax, fabs(tilde[k][v]));
         }
     // exact early exit (tvb_keeps): uniform and near-uniform regions skip
     // the decompositions
     if (tvb_keeps<Real>(mean, gamma, tmax, fmin(fmin(thrk[0], thrk[1]), thrk[2]))) return false;
     // the mean's velocity, sound speed and enthalpy (the eigenvectors below)
-    const Real gm1 = gamma - Real(1), ir = rcp_(mean[0]), vx = mean[1] * ir, vy = mean[2] * ir;
-    const Real k2 = Real(0.5) * (vx * vx + vy * vy);
-    const Real p = gm1 * (mean[3] - mean[0] * k2), H = (mean[3] + p) * ir;
+    const Real gm1 = add_(gamma, Real(-1)), ir = rcp_(mean[0]), vx = mul_(mean[1], ir), vy = mul_(mean[2], ir);
+    const Real k2 = mul_(Real(0.5), fma(vx, vx, mul_(vy, vy)));
+    const Real p = mul_(gm1, fma(-mean[0], k2, mean[3])), H = mul_(add_(mean[3], p), ir);
     Real c, ic;
-    lengths_(gamma * p * ir, c, ic);
-    const Real b1 = gm1 * (ic * ic), b2 = b1 * k2;
+    lengths_(mul_(mul_(gamma, p), ir), c, ic);
+    const Real b1 = mul_(gm1, mul_(ic, ic)), b2 = mul_(b1, k2);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         if ((k == 0 ? cn.x : (k == 1 ? cn.y : cn.z)) >= 0) continue;
         // ghost mean across a boundary edge, mirrored about the unit normal
         // of edge k (N_k / area = 2(r0+r1), -2 r0, -2 r1)
         const int tag = ((unsigned)cn.w >> (6 + 2 * k)) & 3u;
-        const double Nx = k == 0 ? r0.x + r1.x : (k == 1 ? -r0.x : -r1.x);
-        const double Ny = k == 0 ? r0.y + r1.y : (k == 1 ? -r0.y : -r1.y);
+        const double Nx = k == 0 ? add_(r0.x, r1.x) : (k == 1 ? -r0.x : -r1.x);
+        const double Ny = k == 0 ? add_(r0.y, r1.y) : (k == 1 ? -r0.y : -r1.y);
         double len, il;
-        roots_f64(Nx * Nx + Ny * Ny, len, il);
+        roots_f64(fma(Nx, Nx, mul_(Ny, Ny)), len, il);
         const Real far[4] = {(Real)farp[0], (Real)farp[1], (Real)farp[2], (Real)farp[3]};
-        ghost<Real>(tag, mean, far, (Real)(Nx * il), (Real)(Ny * il), near[k]);
+        ghost<Real>(tag, mean, far, (Real)mul_(Nx, il), (Real)mul_(Ny, il), near[k]);
     }
     bool limited = false;
     Real delta[3][4];
@@ -628,20 +628,20 @@ __device__ __noinline__ bool limit_modes(double2 r0, double2 r1, int4 cn, const 
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
             const Real nj = third ? near[(k + 2) % 3][v] : near[(k + 1) % 3][v];
-            dbar[v] = Real(1.5) * (al * (near[k][v] - mean[v]) + be * (nj - mean[v]));
+            dbar[v] = mul_(Real(1.5), fma(al, add_(near[k][v], -mean[v]), mul_(be, add_(nj, -mean[v]))));
         }
         // characteristic components in direction n at the mean: with
         // s = b2 a0 - b1 (v.m - aE) and d = (q a0 - m.n) / c they are
         // (s + d) / 2, a0 - s, -q_t a0 - n_y m_x + n_x m_y and (s - d) / 2
-        const Real q = vx * nx + vy * ny, qt = vy * nx - vx * ny;
+        const Real q = fma(vx, nx, mul_(vy, ny)), qt = fma(vy, nx, -mul_(vx, ny));
         Real wl[4], w[2][4];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const Real* a = i ? dbar : tilde[k];
-            const Real s = b2 * a[0] - b1 * (vx * a[1] + vy * a[2] - a[3]);
-            const Real d = (q * a[0] - (a[1] * nx + a[2] * ny)) * ic;
-            w[i][0] = Real(0.5) * (s + d), w[i][1] = a[0] - s, w[i][2] = nx * a[2] - ny * a[1] - qt * a[0],
-            w[i][3] = Real(0.5) * (s - d);
+            const Real s = fma(b2, a[0], -mul_(b1, fma(vx, a[1], fma(vy, a[2], -a[3]))));
+            const Real d = mul_(fma(q, a[0], -fma(a[1], nx, mul_(a[2], ny))), ic);
+            w[i][0] = mul_(Real(0.5), add_(s, d)), w[i][1] = add_(a[0], -s);
+            w[i][2] = fma(nx, a[2], -fma(ny, a[1], mul_(qt, a[0]))), w[i][3] = mul_(Real(0.5), add_(s, -d));
         }
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -653,35 +653,35 @@ __device__ __noinline__ bool limit_modes(double2 r0, double2 r1, int4 cn, const 
             limited = limited || wl[r] != wt;
         }
         // back through the right eigenvectors
-        const Real sum = wl[0] + wl[1] + wl[3], dif = (wl[3] - wl[0]) * c;
+        const Real sum = add_(add_(wl[0], wl[1]), wl[3]), dif = mul_(add_(wl[3], -wl[0]), c);
         delta[k][0] = sum;
-        delta[k][1] = vx * sum + nx * dif - ny * wl[2];
-        delta[k][2] = vy * sum + ny * dif + nx * wl[2];
-        delta[k][3] = H * (wl[0] + wl[3]) + q * dif + k2 * wl[1] + qt * wl[2];
+        delta[k][1] = fma(vx, sum, fma(nx, dif, -mul_(ny, wl[2])));
+        delta[k][2] = fma(vy, sum, fma(ny, dif, mul_(nx, wl[2])));
+        delta[k][3] = fma(H, add_(wl[0], wl[3]), fma(q, dif, fma(k2, wl[1], mul_(qt, wl[2]))));
     }
     if (!limited) return false;
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
-        Real s = delta[0][v] + delta[1][v] + delta[2][v];
+        const Real s = add_(add_(delta[0][v], delta[1][v]), delta[2][v]);
         if (s != Real(0)) {
             Real pos = Real(0), neg = Real(0);
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                pos += fmax(Real(0), delta[k][v]);
-                neg += fmax(Real(0), -delta[k][v]);
+                pos = add_(pos, fmax(Real(0), delta[k][v]));
+                neg = add_(neg, fmax(Real(0), -delta[k][v]));
             }
             // theta+ = min(1, neg / pos), theta- = min(1, pos / neg): one of them is 1
-            const Real lo = fmin(pos, neg), hi = fmax(pos, neg), th = lo * rcp_(hi);
+            const Real lo = fmin(pos, neg), hi = fmax(pos, neg), th = mul_(lo, rcp_(hi));
             const Real tp = pos > neg ? th : Real(1), tn = neg > pos ? th : Real(1);
 #pragma unroll
             for (int k = 0; k < 3; ++k)
-                delta[k][v] = tp * fmax(Real(0), delta[k][v]) - tn * fmax(Real(0), -delta[k][v]);
+                delta[k][v] = fma(tp, fmax(Real(0), delta[k][v]), -mul_(tn, fmax(Real(0), -delta[k][v])));
         }
     }
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
-        m1[v] = tb.minv[0][0] * delta[0][v] + tb.minv[0][1] * delta[1][v] + tb.minv[0][2] * delta[2][v];
-        m2[v] = tb.minv[1][0] * delta[0][v] + tb.minv[1][1] * delta[1][v] + tb.minv[1][2] * delta[2][v];
+        m1[v] = fma(tb.minv[0][0], delta[0][v], fma(tb.minv[0][1], delta[1][v], mul_(tb.minv[0][2], delta[2][v])));
+        m2[v] = fma(tb.minv[1][0], delta[0][v], fma(tb.minv[1][1], delta[1][v], mul_(tb.minv[1][2], delta[2][v])));
     }
     return true;
 }

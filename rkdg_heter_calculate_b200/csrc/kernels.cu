@@ -7,9 +7,10 @@
 // gradients, forms the edge traces and the Riemann flux at the Gauss points
 // of every edge once per tile, and applies the SSP-RK stage update in its
 // epilogue.  Nothing but the state is written to HBM: traces, fluxes and
-// residuals live in registers and shared memory.  This file also holds the
-// physics helpers, the TVB limiter, the CFL/step kernels and the boundary
-// conversions.
+// residuals live in registers and shared memory.  Device functions common to
+// the CUDA sources are in device.cuh; solves that fit on the device run whole
+// steps in one launch (resident.cuh).  This file also holds the limiter's
+// kernel, the CFL/step kernels and the boundary conversions.
 //
 // HBM layout (element-interleaved packs for 128-bit accesses):
 //   state  : row r = 4*i + v (basis i, variable v), packs of W = 16/sizeof(Real)

@@ -10,7 +10,7 @@
 // What bounds it: latency at 12 warps per SM (168 registers): the FP64 pipe
 // is busy 40 % and issue 34 % of the time.  980,000 P2 HLLC triangles:
 // 0.723 ms per step with IEEE divides and roots, two-sided fluxes and
-// 32-byte traces, 0.591 as it is (7-point LLF 0.683 -> 0.556).
+// 32-byte traces, 0.587 as it is (7-point LLF 0.683 -> 0.547).
 //
 // Every sum of products is spelled as fused multiply-adds and roundings that
 // the compiler may not contract (add_, mul_), so each kernel built from these

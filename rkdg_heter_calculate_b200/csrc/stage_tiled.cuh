@@ -1,5 +1,5 @@
 // Tile-staged fused stage kernel (included by kernels.cu): the staging
-// pipeline and the FP32 kernel (FP64: stage_pair.cuh).
+// pipeline and the FP32 kernel (FP64: stage_fp64.cuh).
 //
 // A tile is up to BT consecutive (locality-ordered) elements of one
 // solve; its descriptor names the element range, the solve, the polynomial
@@ -12,10 +12,9 @@
 //            its lower-index side; every halo and boundary edge from the
 //            in-tile side), spread evenly over the threads; the physical
 //            flux (normal scaled by the edge length) overwrites the
-//            computing side's trace slot.
-//   phase C  each thread adds its three edges' fluxes (its own slot, or the
-//            negated flux of the in-tile neighbour that computed it) to the
-//            residual and applies the stage update.
+//            computing side's trace slot, its negation the other side's.
+//   phase C  each thread adds the fluxes in its own nine (P1: six) slots to
+//            the residual and applies the stage update.
 // The kernel loops over tiles (tile = blockIdx.x + k * gridDim.x), so one
 // launch serves a single solve (one CTA per tile) or a persistent pass over
 // the packed tiles of many solves of uneven size and mixed order, each with
@@ -29,7 +28,8 @@
 // that needs no other is issued first, nobody waits for the thread that
 // issues the copies, the reference state comes from a table, and the edge
 // tables are loaded once per CTA: 980,000 P2 triangles 0.288 -> 0.263 ms per
-// step in FP32 and 0.310 -> 0.289 in FP32C, P1 with LLF 0.171 -> 0.158.
+// step in FP32 and 0.310 -> 0.289 in FP32C, P1 with LLF 0.171 -> 0.158; with
+// overlapping launches and branch-free flux stores 0.254, 0.277 and 0.148.
 //
 // Staging pipeline: a tile's own state rows are contiguous 16-byte rows in
 // HBM (pack p of element e at (p ld + e) 16), so one thread moves them into
@@ -112,7 +112,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint64
 // state rows by bulk copy (SROWS rows of 16 bytes per element); once phase A
 // has read them, the halo neighbours' states by 16-byte gathers ([SROWS][hm]
 // rows).  Each halo thread then overwrites its own neighbour's first rows
-// with that neighbour's traces (and mean: put_htr), which phase B reads, and
+// with that neighbour's traces (and mean), which phase B reads, and
 // the next tile's rows are copied in after phase B.  This keeps an FP32 CTA
 // within the shared memory of six per SM (P2) and an FP64 one within that of
 // three (P2) or four (P1).  J^-1 and the edge codes are read per thread (L2
