@@ -390,9 +390,9 @@ int rkdg_server_destroy(rkdg_server* s);
 int rkdg_server_submit(rkdg_server* s, const rkdg_mesh_desc* mesh, int32_t order, const double* U0,
                        double t_final, const double* farfield, int32_t limiter, int64_t* id);
 /* As rkdg_server_submit, with the request's own Riemann flux (RKDG_FLUX_*;
- * rkdg_server_submit uses params->flux).  The loop runs the LLF and the
- * HLLC requests' tiles as two launches per stage on two streams, joined
- * before the next stage. */
+ * rkdg_server_submit uses params->flux).  The loop runs the requests
+ * of each flux and order as a chain of launches of its own; the chains meet
+ * where the loop reads the control blocks. */
 int rkdg_server_submit_method(rkdg_server* s, const rkdg_mesh_desc* mesh, int32_t order, const double* U0,
                               double t_final, const double* farfield, int32_t limiter, int32_t flux,
                               int64_t* id);

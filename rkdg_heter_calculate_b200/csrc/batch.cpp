@@ -40,14 +40,14 @@ struct rkdg_batch {
     StepCtl* ctl = nullptr;
     StepCtl* h_ctl = nullptr;
     cudaStream_t stream = nullptr;
-    cudaStream_t stream2 = nullptr;    // tile order 2: the P1 tiles' launches, forked and joined
+    cudaStream_t stream2 = nullptr;    // tile order 2: the P1 tiles' chain of launches
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     int n2tiles = 0;                   // P2 tiles (the first ones in tile orders 1 and 2)
     cudaGraphExec_t graph = nullptr;   // one step
     cudaGraphExec_t graph_n = nullptr; // kGraphSteps steps (fewer graph launches and boundaries)
     // tile order: 0 = solve order, 1 = P2 tiles first, 2 = P2 tiles first
-    // and the P2 and P1 tiles as two launches of the single-order kernels on
-    // forked streams (mixed packs)
+    // and the P2 and P1 tiles as two chains of the single-order kernels on
+    // two streams (mixed packs)
     int ctas = 0, tile_order = 0, tile = kTile;
     std::vector<HostMesh> topo;  // per solve (internal order): T, neighbours, shared edges, tags
     size_t table_bytes = 0;      // device bytes of the tile tables (rebuilt with the tile size)

@@ -144,7 +144,7 @@ struct rkdg_server {
     double* staging = nullptr;
     StepCtl* h_ctl = nullptr;
     cudaStream_t stream = nullptr;
-    cudaStream_t side[kLists - 1] = {nullptr, nullptr, nullptr};  // lists 1.., forked and joined per stage
+    cudaStream_t side[kLists - 1] = {nullptr, nullptr, nullptr};  // lists 1.., forked and joined per chunk
     cudaEvent_t ev_fork = nullptr, ev_join[kLists - 1] = {nullptr, nullptr, nullptr};
     cudaGraphExec_t graph = nullptr;
     TileArgs tiles[kLists]{};  // per list (flux, order)
