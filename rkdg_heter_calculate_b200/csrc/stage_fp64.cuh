@@ -432,7 +432,10 @@ __global__ void __launch_bounds__(BT, Fp64Occupancy<ORD, BT, LAT>::value)
     unsigned char* stg = smem_raw + SM::stage_offset(ta.max_halo);
     const int ntiles = ta.ntiles_dev ? *ta.ntiles_dev : ta.ntiles;
     int tile = blockIdx.x;
-    if (tile >= ntiles) return;
+    if (tile >= ntiles) {  // a launch without a tile also completes only after the ones ahead of it
+        grid_dependency_wait();
+        return;
+    }
     const int tid = threadIdx.x;
     int4 d0 = __ldg(ta.desc + 2 * tile), d1 = __ldg(ta.desc + 2 * tile + 1);
     grid_dependents_launch();

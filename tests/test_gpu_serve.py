@@ -167,3 +167,25 @@ def test_engine_failure_fails_every_request_and_is_reported():
         with pytest.raises(capi.RkdgError) as e:
             submit(srv, reqs[3])
         assert e.value.code == capi.RKDG_ERR_CUDA
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp32c", "fp64"])
+def test_limited_requests_after_their_list_was_idle(precision):
+    """The limited requests' tile lists are empty for some hundred chunks while
+    others run, then hold one request after another: the limiter's arrival
+    counts and tile flags of an idle list must stay as they were, or tiles go
+    unlimited.  Each result equals the solve alone."""
+    reqs = requests()
+    vortices, limited = reqs[:4], reqs[4:]
+    ref = [solo(r, precision) for r in limited]
+    with Server(256 * MB, max_slots=8, precision=precision, **SERVER) as srv:
+        for _ in range(3):
+            for r in [submit(srv, v) for v in vortices]:
+                assert srv.wait(r).status == DONE
+            running = submit(srv, vortices[0])
+            for k, r in enumerate(limited):
+                res = srv.wait(submit(srv, r))
+                assert res.steps == ref[k][2]
+                np.testing.assert_array_equal(res.state, ref[k][0], err_msg=f"limited request {k}")
+            srv.wait(running)
+        assert srv.timing()["chunks"] > 100
