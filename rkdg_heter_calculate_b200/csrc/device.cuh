@@ -174,15 +174,18 @@ static void upload_module_tables(int nq, int ng) {
 }
 
 // --------------------------------------------------------- state packs --
+// States are read with ordinary loads: a kernel launched early
+// (launch_dependent) is alive while the one ahead writes them, and the
+// read-only path (__ldg, or a const __restrict__ kernel parameter) is for
+// memory that nothing writes in a kernel's lifetime.
 template <typename Real, int NB>
-__device__ __forceinline__ void load_state(const Real* __restrict__ U, int ld, int e,
-                                           Real u[NB][4]) {
+__device__ __forceinline__ void load_state(const Real* U, int ld, int e, Real u[NB][4]) {
     if constexpr (sizeof(Real) == 8) {
         const double2* p = reinterpret_cast<const double2*>(U);
 #pragma unroll
         for (int i = 0; i < NB; ++i) {
-            double2 a = __ldg(p + (size_t)(2 * i) * ld + e);
-            double2 b = __ldg(p + (size_t)(2 * i + 1) * ld + e);
+            double2 a = p[(size_t)(2 * i) * ld + e];
+            double2 b = p[(size_t)(2 * i + 1) * ld + e];
             u[i][0] = a.x;
             u[i][1] = a.y;
             u[i][2] = b.x;
@@ -192,7 +195,7 @@ __device__ __forceinline__ void load_state(const Real* __restrict__ U, int ld, i
         const float4* p = reinterpret_cast<const float4*>(U);
 #pragma unroll
         for (int i = 0; i < NB; ++i) {
-            float4 a = __ldg(p + (size_t)i * ld + e);
+            float4 a = p[(size_t)i * ld + e];
             u[i][0] = a.x;
             u[i][1] = a.y;
             u[i][2] = a.z;
@@ -202,7 +205,7 @@ __device__ __forceinline__ void load_state(const Real* __restrict__ U, int ld, i
 }
 
 template <typename Real, int NB>
-__device__ __forceinline__ void load_mean(const Real* __restrict__ U, int ld, int e, Real m[4]) {
+__device__ __forceinline__ void load_mean(const Real* U, int ld, int e, Real m[4]) {
     Real u[1][4];
     load_state<Real, 1>(U, ld, e, u);
     m[0] = u[0][0], m[1] = u[0][1], m[2] = u[0][2], m[3] = u[0][3];
@@ -225,30 +228,23 @@ struct Ref4 {
     double v[4];
 };
 
-template <typename Real, int NB>
-__device__ __forceinline__ void store_state(Real* __restrict__ U, int ld, int e,
-                                            const Real u[NB][4]) {
-    if constexpr (sizeof(Real) == 8) {
-        double2* p = reinterpret_cast<double2*>(U);
+// the modes I0..NB-1 of a state
+template <typename Real, int I0, int NB>
+__device__ __forceinline__ void store_rows(Real* U, int ld, int e, const Real u[NB][4]) {
 #pragma unroll
-        for (int i = 0; i < NB; ++i) {
+    for (int i = I0; i < NB; ++i) {
+        if constexpr (sizeof(Real) == 8) {
+            double2* p = reinterpret_cast<double2*>(U);
             p[(size_t)(2 * i) * ld + e] = make_double2(u[i][0], u[i][1]);
             p[(size_t)(2 * i + 1) * ld + e] = make_double2(u[i][2], u[i][3]);
+        } else {
+            reinterpret_cast<float4*>(U)[(size_t)i * ld + e] = make_float4(u[i][0], u[i][1], u[i][2], u[i][3]);
         }
-    } else {
-        float4* p = reinterpret_cast<float4*>(U);
-#pragma unroll
-        for (int i = 0; i < NB; ++i) p[(size_t)i * ld + e] = make_float4(u[i][0], u[i][1], u[i][2], u[i][3]);
     }
 }
-
-// rows I0..NB-1 of a state (the FP32 form's one 16-byte pack per basis function)
-template <typename Real, int I0, int NB>
-__device__ __forceinline__ void store_rows(Real* __restrict__ U, int ld, int e, const Real u[NB][4]) {
-    static_assert(sizeof(Real) == 4, "one pack per row: FP32 states");
-    float4* p = reinterpret_cast<float4*>(U);
-#pragma unroll
-    for (int i = I0; i < NB; ++i) p[(size_t)i * ld + e] = make_float4(u[i][0], u[i][1], u[i][2], u[i][3]);
+template <typename Real, int NB>
+__device__ __forceinline__ void store_state(Real* U, int ld, int e, const Real u[NB][4]) {
+    store_rows<Real, 0, NB>(U, ld, e, u);
 }
 
 // ------------------------------------------------------------- physics --

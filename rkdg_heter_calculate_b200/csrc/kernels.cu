@@ -112,7 +112,7 @@ __global__ void step_begin_kernel(StepCtl* ctls, int n, int chain) {
 }
 
 template <typename Real, int NB>
-__device__ __forceinline__ void limit_element(int e, int ld, Real* __restrict__ U,
+__device__ __forceinline__ void limit_element(int e, int ld, Real* U,
                                               const int4* __restrict__ conn,
                                               const void* __restrict__ limv,
                                               const double* __restrict__ jinv, double gamma,
@@ -143,13 +143,12 @@ __device__ __forceinline__ void limit_element(int e, int ld, Real* __restrict__ 
     Real out[NB][4];
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
-        out[0][v] = u[0][v];
         out[1][v] = m1[v];
         out[2][v] = m2[v];
 #pragma unroll
         for (int i = 3; i < NB; ++i) out[i][v] = Real(0);
     }
-    store_state<Real, NB>(U, ld, e, out);
+    store_rows<Real, 1, NB>(U, ld, e, out);  // the mean stays: other blocks read it
 }
 
 // One tile of the limiter (all threads of the CTA): tiles of solves whose
@@ -157,11 +156,11 @@ __device__ __forceinline__ void limit_element(int e, int ld, Real* __restrict__ 
 // skipped; P1 and P2 tiles limit their P1 part (P2 tiles drop their
 // quadratic modes where limited).
 template <typename Real>
-__device__ __forceinline__ void limit_tile(const TileArgs& ta, int tile, int ld, Real* __restrict__ U,
+__device__ __forceinline__ void limit_tile(const TileArgs& ta, int tile, int ld, Real* U,
                                            const int4* __restrict__ conn, const void* __restrict__ lim,
                                            const double* __restrict__ jinv, const int* __restrict__ flags,
                                            const double* __restrict__ refs, double gamma, double tvb_m, int cfg1,
-                                           int cfg2, const StepCtl* __restrict__ ctl) {
+                                           int cfg2, const StepCtl* ctl) {
     const int4 d0 = __ldg(ta.desc + 2 * tile);
     if ((flags && !flags[d0.z]) || (ctl && ctl[d0.z].done)) return;
     const double* f = refs + 4 * d0.z;
@@ -182,7 +181,7 @@ __device__ __forceinline__ void limit_tile(const TileArgs& ta, int tile, int ld,
 // element fails tvb_keeps) and cost nothing.
 template <typename Real>
 __global__ void __launch_bounds__(kAuxBlock) tiled_limiter_kernel(const TileArgs ta, int ld,
-                                                              Real* __restrict__ U,
+                                                              Real* U,
                                                               const int4* __restrict__ conn,
                                                               const void* __restrict__ lim,
                                                               const double* __restrict__ jinv,
@@ -190,7 +189,7 @@ __global__ void __launch_bounds__(kAuxBlock) tiled_limiter_kernel(const TileArgs
                                                               const double* __restrict__ refs,
                                                               double gamma, double tvb_m,
                                                               int cfg1, int cfg2,
-                                                              const StepCtl* __restrict__ ctl,
+                                                              const StepCtl* ctl,
                                                               int* __restrict__ tile_flags,
                                                               int* __restrict__ tile_list, int tile_cap) {
     grid_dependents_launch();

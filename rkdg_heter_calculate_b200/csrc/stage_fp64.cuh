@@ -336,7 +336,7 @@ __device__ __forceinline__ bool tile_stage_fp64(const StageArgs& a, const TileAr
         const double2* U0 = static_cast<const double2*>(a.U0) + ee;
 #pragma unroll
         for (int r = 0; r < 2 * NB; ++r) {
-            const double2 x = __ldg(Uin + (size_t)r * a.ld);  // stored values (L2 hits)
+            const double2 x = Uin[(size_t)r * a.ld];  // stored values (L2 hits)
             const double2 y = U0[(size_t)r * a.ld];
             if (r == 0) u0m[0] = y.x;
             if (r == 1) u0m[1] = y.y;
@@ -346,7 +346,7 @@ __device__ __forceinline__ bool tile_stage_fp64(const StageArgs& a, const TileAr
     } else {
 #pragma unroll
         for (int r = 0; r < 2 * NB; ++r) {
-            const double2 x = __ldg(Uin + (size_t)r * a.ld);
+            const double2 x = Uin[(size_t)r * a.ld];
             double2& v = R[r / 2][r % 2];
             v = make_double2(mul_(cb, fma(dt, v.x, x.x)), mul_(cb, fma(dt, v.y, x.y)));
         }

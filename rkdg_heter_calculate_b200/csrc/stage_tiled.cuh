@@ -512,7 +512,7 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
     const bool active = tid < d0.y;
     const int ee = active ? e : e0;
     const int sx = active ? tid : 0;  // staging row index
-    const Real* __restrict__ U = static_cast<const Real*>(a.U);
+    const Real* U = static_cast<const Real*>(a.U);
     const Real gamma = (Real)a.gamma, gm1 = gamma - Real(1);
     // traces and fluxes in deviation form about the reference state; a
     // stored mean is the deviation from it
@@ -613,7 +613,7 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
     // every own slot now holds the outward flux of its edge point
     project32<NB, NG, BT>(t2, s_tr, R);
 
-    Real* __restrict__ Uout = static_cast<Real*>(a.Unew);
+    Real* Uout = static_cast<Real*>(a.Unew);
     if (MODE == MODE_RESIDUAL) {
         const Real sc = (Real)det;
 #pragma unroll
@@ -629,9 +629,13 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
     // RKDG_FP32C (comp): row 0 is updated in FP64 below, not here
     constexpr bool comp = (MODE & MODE_STAGE_COMP) != 0;
     load_state<Real, NB>(U, a.ld, ee, u);  // stored values (L2 hit)
+    const size_t lr = comp ? (size_t)a.lo_row * a.ld : 0;
+    float4 l = make_float4(0.f, 0.f, 0.f, 0.f), l0 = l;
+    if constexpr (comp) l = reinterpret_cast<const float4*>(a.U)[lr + ee];
     if (a.U0 != nullptr) {
         Real u0[NB][4];
         load_state<Real, NB>(static_cast<const Real*>(a.U0), a.ld, ee, u0);
+        if constexpr (comp) l0 = reinterpret_cast<const float4*>(a.U0)[lr + ee];
 #pragma unroll
         for (int i = comp ? 1 : 0; i < NB; ++i) update_row32(u[i], u0[i], dt, cb, R[i]);
 #pragma unroll
@@ -648,10 +652,6 @@ __device__ __forceinline__ bool tile_stage(const StageArgs& a, const TileArgs& t
         // high and a low float, so the mean's storage rounding does not
         // accumulate over the stages.
         if (active) store_rows<Real, 1, NB>(Uout, a.ld, e, R);
-        const size_t lr = (size_t)a.lo_row * a.ld;
-        const float4 l = __ldg(reinterpret_cast<const float4*>(a.U) + lr + ee);
-        float4 l0 = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (a.U0 != nullptr) l0 = __ldg(reinterpret_cast<const float4*>(a.U0) + lr + ee);
         const float lv[4] = {l.x, l.y, l.z, l.w}, l0v[4] = {l0.x, l0.y, l0.z, l0.w};
         float nl[4];
         update_mean32c(u[0], lv, u0m, l0v, mul_(dtd, det), a.b, R[0], nl);

@@ -57,3 +57,20 @@ def test_no_path_leaves_before_the_wait(name):
     assert "grid_dependency_wait()" in text
     for m in re.finditer(r"\breturn\b", text):
         assert "grid_dependency_wait()" in text[: m.start()], text[max(0, m.start() - 80): m.end()]
+
+
+# arguments of __ldg: the tables of a mesh, a rule or a solve, which no kernel writes
+TABLES = ("ta.", "&ta.", "jinv2 ", "j2 ", "conn ", "lim ", "&g[", "t)", "t +")
+
+
+def test_written_memory_is_not_read_through_the_read_only_path():
+    """A kernel that starts early is alive while the one ahead writes the
+    states and control blocks; the read-only path is for memory that nothing
+    writes in the kernel's lifetime, and its loads may move above the wait."""
+    for name in ["kernels.cu", "device.cuh", "stage_tiled.cuh", "stage_fp64.cuh"]:
+        for m in re.finditer(r"__ldg\(([^;]*)", source(name)):
+            assert m.group(1).startswith(TABLES), (name, m.group(0)[:60])
+    limiter = re.search(r"tiled_limiter_kernel\(.*?\{", source("kernels.cu"), re.S).group(0)
+    for p in limiter.split(","):
+        if re.search(r"\b(U|ctl)$", p.strip()):
+            assert "__restrict__" not in p, p
