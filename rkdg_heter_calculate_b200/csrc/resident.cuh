@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(NT, (sizeof(Real) == 8 ? 256 : 512) / NT) resi
             }
             if (reads) {  // the neighbour's traces on the shared edge, and its mean
                 uint4 v[SM::TR];
-                ok = collect_rows<SM::TR>(xt + in, ns, ep, v);
+                ok = collect_rows<SM::TR>(xt + in, ns, ep, v) && ok;  // (a lost mean of the stage before counts too)
 #pragma unroll
                 for (int r = 0; r < SM::TR; ++r) bits_row(v[r], s_htr[r * HM + el]);
             }
