@@ -21,7 +21,8 @@
 // needs the maximum wave speed of all tiles: each adds its own to the step's
 // slot and counts itself in, and the sum is awaited only beside the flux tasks
 // of the next step's first stage.  Every wait is bounded (kStageWaitNs) and
-// reports through the control block, as the staging waits do.
+// reports through the control block, as the staging waits do, and ends the
+// solve there.
 //
 // The edges other tiles read are formed and published first (from the table
 // in shared memory, by a runtime edge), the tile's own traces after them.  With
@@ -559,8 +560,12 @@ finished:
         if (tid < 2) a.mon[tid] = 0ull;
     }
     return;
-lost:  // a wait ran out: report and leave (the other tiles' waits run out too)
-    if (tid == 0) atomicOr(&a.ctl->error, 2);
+lost:  // a wait ran out: report and leave (the other tiles' waits run out too);
+       // launches queued behind find the solve done and leave at once
+    if (tid == 0) {
+        atomicOr(&a.ctl->error, 2);
+        atomicExch(&a.ctl->done, 1);
+    }
 }
 
 // ------------------------------------------------------------- host --

@@ -26,3 +26,10 @@ def launches(tmp_path_factory):
 def test_a_lost_mean_is_reported(launches):
     error, _, _, ms = launches[0]
     assert error == 2 and 1500 < ms < 10000, launches
+
+
+def test_launches_behind_a_lost_wait_leave_at_once(launches):
+    """A whole advance is queued without a read-back in between: none of the
+    launches behind the failed one may wait again, or step on from its state."""
+    (_, done, steps, _), (error, _, steps2, ms) = launches
+    assert done == 1 and steps == steps2 == 0 and error == 2 and ms < 500, launches
