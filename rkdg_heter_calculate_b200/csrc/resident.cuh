@@ -363,6 +363,7 @@ __global__ void __launch_bounds__(NT, (sizeof(Real) == 8 ? 256 : 512) / NT) resi
                     stop = 1;
                     bad_dt = 1;
                     done = 1;
+                    add_release(a.count + step, 1u);  // (it has read the control block and the sums)
                 }
                 if (stop == 0) {
                     t = last ? t_final : t + dt;
@@ -540,8 +541,9 @@ finished:
         for (int r = 0; r < SR; ++r) U[r * ld] = s_u[r * BT + el];
     if (blockIdx.x == 0 && tid == CT) {
         StepCtl* c = a.ctl;
+        // the block changes only after every tile has read it
+        if (steps + bad_dt > 0 && !wait_count(a.count + steps + bad_dt - 1, gridDim.x)) ok = false;
         if (steps > 0) {
-            if (!wait_count(a.count + steps - 1, gridDim.x)) ok = false;
             c->wave_bits = __ldcg(a.wave + steps - 1);
             c->mon_bits[0] = a.monitor ? __ldcg(a.mon + 0) : 0ull;
             c->mon_bits[1] = a.monitor ? __ldcg(a.mon + 1) : 0ull;
@@ -554,8 +556,9 @@ finished:
     }
     if (__syncthreads_or(!ok)) goto lost;
     // every tile has counted itself into the last step, so none will read the
-    // sums again: zero for the next launch (after an error the host clears them)
-    if (blockIdx.x == 0 && !s_stop) {
+    // sums again: zero for the next launch (after an error the host clears
+    // them as well)
+    if (blockIdx.x == 0) {
         for (int i = tid; i < a.nsteps; i += NT) a.wave[i] = 0ull, a.count[i] = 0u;
         if (tid < 2) a.mon[tid] = 0ull;
     }

@@ -129,3 +129,19 @@ def test_resident_solves_in_several_threads():
         t.join()
     for out in together:
         np.testing.assert_array_equal(out, alone[0])
+
+
+@pytest.mark.parametrize("n", [40, 97])  # 25 and 148 tiles
+def test_resident_reports_a_bad_first_time_step(n):
+    """Every tile stops at the first step's dt; whichever block comes first or
+    last, that is a state error, not a wait that ran out."""
+    from rkdg_heter_calculate_b200.capi import RkdgError
+
+    mesh = ordered(meshgen.periodic_structured(n, n, jitter=0.15, seed=2))
+    s = CUDARkdgSolver(mesh, farfield=FAR, order=2, nq=6, ng=3, flux="hllc", cfl=0.2)
+    s.setFreedom(start(mesh, 6, FAR, "vortex"), basis="native")
+    for _ in range(50):
+        with pytest.raises(RkdgError) as e:
+            s.step(float("inf"))
+        assert e.value.code == 4
+    s.close()
