@@ -8,10 +8,11 @@
 
 #include <algorithm>
 #include <cstdint>
-#include <mutex>
+#include <map>
 #include <string>
 #include <type_traits>
 
+#include "per_device.hpp"
 #include "rkdg_internal.hpp"
 #include "roots.cuh"
 

@@ -406,29 +406,31 @@ __global__ void __launch_bounds__(kTotBlock) totals_final_kernel(int n, const do
 // ----------------------------------------------------------- launchers --
 void upload_tables(int nq, int ng) { upload_module_tables(nq, ng); }
 
+int current_device() {
+    int dev = 0;
+    RKDG_CUDA_TRY(cudaGetDevice(&dev));
+    return dev;
+}
+
+// An attribute of the current device, asked for once on each (none is zero).
+static int device_attribute(PerDevice<int>& kept, cudaDeviceAttr attr) {
+    const int dev = current_device();
+    return kept.use(dev, [&](int& v) {
+        if (v == 0) RKDG_CUDA_TRY(cudaDeviceGetAttribute(&v, attr, dev));
+        return v;
+    });
+}
+
 // The device's largest opt-in dynamic + static shared memory per CTA, less
 // the kernels' static shared memory (barrier, maxima, dt, tables).
 size_t smem_limit() {
-    static int limit = 0;
-    if (limit == 0) {
-        int dev = 0, v = 0;
-        RKDG_CUDA_TRY(cudaGetDevice(&dev));
-        RKDG_CUDA_TRY(cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        limit = v;
-    }
-    return (size_t)limit - 1024;
+    static PerDevice<int> limit;
+    return (size_t)device_attribute(limit, cudaDevAttrMaxSharedMemoryPerBlockOptin) - 1024;
 }
 
-
 int sm_count() {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0, v = 0;
-        RKDG_CUDA_TRY(cudaGetDevice(&dev));
-        RKDG_CUDA_TRY(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev));
-        n = v;
-    }
-    return n;
+    static PerDevice<int> n;
+    return device_attribute(n, cudaDevAttrMultiProcessorCount);
 }
 
 namespace {
@@ -471,28 +473,31 @@ size_t prepare_tiled(int max_halo) {
     constexpr auto kernel = stage_kernel<Real, NQ2, FLUX, MODE, ORD, BT, LAT>();
     // dynamic + static shared memory above 48 KB needs the opt-in.  Per
     // instantiation; raised when a context with a larger halo appears.
-    static size_t configured = 0;
-    if (configured == 0)  // give shared memory the whole carveout
-        RKDG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                           (int)cudaSharedmemCarveoutMaxShared));
-    if (smem > configured) {
-        RKDG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        configured = smem;
-    }
+    static PerDevice<size_t> opt_in;
+    opt_in.use(current_device(), [&](size_t& configured) {
+        if (configured == 0)  // give shared memory the whole carveout
+            RKDG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                               (int)cudaSharedmemCarveoutMaxShared));
+        if (smem > configured) {
+            RKDG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            configured = smem;
+        }
+    });
     return smem;
 }
 
 template <typename Real, int NQ2, int FLUX, int MODE, int ORD, int BT>
 int occupancy_tiled(int max_halo) {
     const size_t smem = prepare_tiled<Real, NQ2, FLUX, MODE, ORD, BT>(max_halo);
-    thread_local size_t of = 0;  // the last answer, per instantiation and thread
-    thread_local int n = 0;
-    if (of != smem) {
+    static PerDevice<std::map<size_t, int>> answers;  // by shared memory
+    return answers.use(current_device(), [&](std::map<size_t, int>& known) {
+        const auto it = known.find(smem);
+        if (it != known.end()) return it->second;
         constexpr auto kernel = stage_kernel<Real, NQ2, FLUX, MODE, ORD, BT>();
+        int n = 0;
         RKDG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, BT, smem));
-        of = smem;
-    }
-    return n;
+        return known[smem] = n;
+    });
 }
 
 template <typename Real, int NQ2, int FLUX, int MODE, int ORD, int BT, int LAT = 0>

@@ -583,19 +583,20 @@ struct ResidentForm {
     template <int NT>
     static int fit(int max_halo) {
         if (max_halo > kTile || SM::bytes(max_halo) > smem_limit()) return 0;
-        thread_local int of = -1, tiles = 0;  // the last answer
-        if (of == max_halo) return tiles;
-        static std::once_flag once;  // the whole opt-in size, whatever halo lists come later
-        std::call_once(once, [] {
-            RKDG_CUDA_TRY(cudaFuncSetAttribute(kernel<NT>(), cudaFuncAttributePreferredSharedMemoryCarveout,
-                                               (int)cudaSharedmemCarveoutMaxShared));
-            RKDG_CUDA_TRY(cudaFuncSetAttribute(kernel<NT>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem_limit()));
+        static PerDevice<std::map<int, int>> answers;  // by halo size
+        return answers.use(current_device(), [&](std::map<int, int>& known) {
+            if (known.empty()) {  // the whole opt-in size, whatever halo lists come later
+                RKDG_CUDA_TRY(cudaFuncSetAttribute(kernel<NT>(), cudaFuncAttributePreferredSharedMemoryCarveout,
+                                                   (int)cudaSharedmemCarveoutMaxShared));
+                RKDG_CUDA_TRY(cudaFuncSetAttribute(kernel<NT>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)smem_limit()));
+            }
+            const auto it = known.find(max_halo);
+            if (it != known.end()) return it->second;
+            int n = 0;
+            RKDG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel<NT>(), NT, SM::bytes(max_halo)));
+            return known[max_halo] = n * sm_count();
         });
-        int n = 0;
-        RKDG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel<NT>(), NT, SM::bytes(max_halo)));
-        of = max_halo;
-        return tiles = n * sm_count();
     }
     static int tiles(int max_halo) { return std::max(fit<256>(max_halo), fit<128>(max_halo)); }
     // 256 threads per tile while the device holds all tiles that way

@@ -303,6 +303,7 @@ bool tiled_fits(int prec, int order, int flux, int max_halo, int tile);
 // resident CTAs per SM of the tiled stage kernel (order 3: mixed pack) for
 // tiles of `tile` elements
 int tiled_max_ctas_per_sm(int prec, int order, int nq, int flux, int max_halo, int tile = kTile);
+int current_device();
 int sm_count();       // SMs of the current device
 size_t smem_limit();  // dynamic shared memory a CTA may use
 // TVB limiter over tiles; flags[solve] (may be null: all on) enables it per
