@@ -24,12 +24,13 @@ __device__ __forceinline__ double rcp_f64(double x) {
     return fma(y, fma(e, e, e), y);
 }
 // sqrt(x) and its reciprocal; 1e-300 keeps the seed finite at x = 0 (the
-// root is then 1e-150) and vanishes in the rounding of any normal argument.
+// root is then 0, its reciprocal some 1e150) and vanishes in the rounding of
+// any argument above 1e-284.
 __device__ __forceinline__ void roots_f64(double x, double& root, double& inv_root) {
     const double a = x + 1e-300;
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-    const double t = a * y;
+    const double t = x * y;
     const double e = fma(-t, y, 1.0);
     const double h = e * fma(0.375, e, 0.5);
     root = fma(t, h, t);

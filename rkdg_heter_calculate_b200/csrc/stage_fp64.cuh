@@ -10,7 +10,7 @@
 // What bounds it: latency at 12 warps per SM (168 registers): the FP64 pipe
 // is busy 40 % and issue 34 % of the time.  980,000 P2 HLLC triangles:
 // 0.723 ms per step with IEEE divides and roots, two-sided fluxes and
-// 32-byte traces, 0.587 as it is (7-point LLF 0.683 -> 0.547).
+// 32-byte traces, 0.585 as it is (7-point LLF 0.683 -> 0.549).
 //
 // Every sum of products is spelled as fused multiply-adds and roundings that
 // the compiler may not contract (add_, mul_), so each kernel built from these
@@ -87,12 +87,11 @@ __device__ __forceinline__ void volume_term(const Tab<double>& tb, const double2
 // with the edge's coefficient alpha (scaled by len), or HLLC (hllc_flux).
 __device__ __forceinline__ void llf_flux(const double uL[4], const double uR[4], double Nx, double Ny, double alpha,
                                          double gm1, double f[4]) {
-    const double irr = rcp_f64(mul_(uL[0], uR[0]));
     double s[4];
 #pragma unroll
     for (int side = 0; side < 2; ++side) {
         const double* u = side ? uR : uL;
-        const double ri = mul_(side ? uL[0] : uR[0], irr);
+        const double ri = rcp_f64(u[0]);
         const double vx = mul_(u[1], ri), vy = mul_(u[2], ri);
         const double p = mul_(gm1, fma(-0.5, fma(u[1], vx, mul_(u[2], vy)), u[3]));
         const double q = fma(vx, Nx, mul_(vy, Ny));
@@ -115,13 +114,14 @@ __device__ __forceinline__ void llf_flux(const double uL[4], const double uR[4],
 //   c (U_K + ex) = S_K (U*_K - U_K),  ex = (0, d_K n, d_K S_M + p_K),
 //   d_K = rho_K (S_K - q_K),  c = S_K (S_M - q_K) / (S_K - S_M),
 // so a warp whose points fall in different wave regions runs one path and
-// only the selected side's physical flux is formed.  The two densities share
-// one reciprocal.
+// only the selected side's physical flux is formed.  (One reciprocal of the
+// product of the densities costs as much as two, 0.587 ms per step against
+// 0.585 on 980,000 triangles, and is out of range where each density alone is
+// not.)
 __device__ __forceinline__ void hllc_flux(const double uL[4], const double uR[4], double nx, double ny, double gamma,
                                           double f[4]) {
     const double gm1 = add_(gamma, -1.0);
-    const double irr = rcp_f64(mul_(uL[0], uR[0]));
-    const double iL = mul_(uR[0], irr), iR = mul_(uL[0], irr);
+    const double iL = rcp_f64(uL[0]), iR = rcp_f64(uR[0]);
     const double vxL = mul_(uL[1], iL), vyL = mul_(uL[2], iL), vxR = mul_(uR[1], iR), vyR = mul_(uR[2], iR);
     const double pL = mul_(gm1, fma(-0.5, fma(uL[1], vxL, mul_(uL[2], vyL)), uL[3]));
     const double pR = mul_(gm1, fma(-0.5, fma(uR[1], vxR, mul_(uR[2], vyR)), uR[3]));
@@ -129,13 +129,15 @@ __device__ __forceinline__ void hllc_flux(const double uL[4], const double uR[4]
     const double cL = sqrt_f64(mul_(mul_(gamma, pL), iL)), cR = sqrt_f64(mul_(mul_(gamma, pR), iR));
     const double SL = fmin(add_(qL, -cL), add_(qR, -cR)), SR = fmax(add_(qL, cL), add_(qR, cR));
     const double dL = mul_(uL[0], add_(SL, -qL)), dR = mul_(uR[0], add_(SR, -qR));
-    const double SM = mul_(fma(dL, qL, fma(-dR, qR, add_(pR, -pL))), rcp_f64(add_(dL, -dR)));
-    const bool sl = SL >= 0.0, sr = SR <= 0.0;
-    const bool left = sl || (!sr && SM >= 0.0);
+    const bool sl = SL >= 0.0, sr = SR <= 0.0, star = !sl && !sr;
+    // (without a star region S_M is not part of the result, and may be NaN:
+    // two states of zero pressure and the same speed have dL = dR = 0)
+    const double SM = star ? mul_(fma(dL, qL, fma(-dR, qR, add_(pR, -pL))), rcp_f64(add_(dL, -dR))) : 0.0;
+    const bool left = sl || (star && SM >= 0.0);
     const double d = left ? dL : dR, p = left ? pL : pR, q = left ? qL : qR, S = left ? SL : SR;
     const double u0 = left ? uL[0] : uR[0], u1 = left ? uL[1] : uR[1], u2 = left ? uL[2] : uR[2],
                  ep = add_(left ? uL[3] : uR[3], p);
-    const double c = (sl || sr) ? 0.0 : mul_(mul_(S, add_(SM, -q)), rcp_f64(add_(S, -SM)));
+    const double c = star ? mul_(mul_(S, add_(SM, -q)), rcp_f64(add_(S, -SM))) : 0.0;
     f[0] = fma(c, u0, mul_(u0, q));
     f[1] = fma(c, fma(d, nx, u1), fma(u1, q, mul_(p, nx)));
     f[2] = fma(c, fma(d, ny, u2), fma(u2, q, mul_(p, ny)));
