@@ -508,13 +508,28 @@ __device__ __forceinline__ double wave_of(const Real m[4], Real gamma, const Rea
 // (tvb_keeps) for it.  Kernels without MODE_LIMITED carry none of that code.
 enum { MODE_STAGE = 0, MODE_RESIDUAL = 1, MODE_STAGE_COMP = 2, MODE_LIMITED = 4 };
 
+// The limiter's reciprocals and roots.  FP32: IEEE, since a limited element is
+// a discontinuous function of them (only the elements that tvb_keeps does not
+// pass pay: 806,400 limited triangles take 20.5 ms per 100 steps either way);
+// FP64: those of the fluxes.
+__device__ __forceinline__ double lim_rcp(double x) { return rcp_f64(x); }
+__device__ __forceinline__ float lim_rcp(float x) { return __frcp_rn(x); }
+__device__ __forceinline__ void lim_lengths(double x, double& len, double& inv) { roots_f64(x, len, inv); }
+__device__ __forceinline__ void lim_lengths(float x, float& len, float& inv) {
+    len = __fsqrt_rn(x);
+    inv = __frcp_rn(len);
+}
+
 // Exact test that the TVB limiter (limit_element) leaves an element unchanged: every
 // row of its left eigenvector matrix has 1-norm at most B (|q|, |q_t| <=
 // |vx| + |vy|, |nx| + |ny| <= 1.5; 1.001 covers rounding), so when B times
 // the largest |P1 midpoint increment| (tilde) is within the smallest TVB
 // threshold, every characteristic increment is kept.  A non-physical mean
 // (NaN bound) fails the test.  The stage kernel applies it to each stage's
-// output per tile, so the limiter can skip whole tiles.
+// output per tile, so the limiter can skip whole tiles.  Its FP32 reciprocal
+// and root are the approximate ones: their error, some 2^-22, is far inside
+// the 1.001, and the IEEE ones in every element of every stage made the limited
+// step 2.5 % slower.
 template <typename Real>
 __device__ __forceinline__ bool tvb_keeps(const Real mean[4], Real gamma, Real tmax, Real thr_min) {
     const Real ir = rcp_(mean[0]), vx = mean[1] * ir, vy = mean[2] * ir;
@@ -544,7 +559,7 @@ __device__ __forceinline__ void tvb_geometry(Real c0x, Real c0y, Real c1x, Real 
         const Real dx = fma(c0x, dxi, mul_(c1x, deta)), dy = fma(c0y, dxi, mul_(c1y, deta));
         const Real r2 = fma(dx, dx, mul_(dy, dy));
         Real rl, irl;
-        lengths_(r2, rl, irl);
+        lim_lengths(r2, rl, irl);
         dirx[k] = mul_(dx, irl);
         diry[k] = mul_(dy, irl);
         thr[k] = mul_(tvb_m, mul_(Real(4), r2));
@@ -588,7 +603,7 @@ __device__ __forceinline__ bool limit_modes(double2 r0, double2 r1, int4 cn, con
     const unsigned pair_bits = ((unsigned)cn.w >> 12) & 7u;
     // the directions and threshold scales in the working precision: FP64
     // for the parity path, FP32 (from the FP64 J^-1 rows) for the FP32 forms
-    const Real idet = rcp_((Real)fma(r0.x, r1.y, -mul_(r0.y, r1.x)));  // det J
+    const Real idet = lim_rcp((Real)fma(r0.x, r1.y, -mul_(r0.y, r1.x)));  // det J
     // columns of J: x_1 - x_0 and x_2 - x_0
     Real dirx[3], diry[3], thrk[3];
     tvb_geometry<Real>(mul_((Real)r1.y, idet), -mul_((Real)r1.x, idet), -mul_((Real)r0.y, idet), mul_((Real)r0.x, idet),
@@ -605,11 +620,11 @@ __device__ __forceinline__ bool limit_modes(double2 r0, double2 r1, int4 cn, con
     // the decompositions
     if (tvb_keeps<Real>(mean, gamma, tmax, fmin(fmin(thrk[0], thrk[1]), thrk[2]))) return false;
     // the mean's velocity, sound speed and enthalpy (the eigenvectors below)
-    const Real gm1 = add_(gamma, Real(-1)), ir = rcp_(mean[0]), vx = mul_(mean[1], ir), vy = mul_(mean[2], ir);
+    const Real gm1 = add_(gamma, Real(-1)), ir = lim_rcp(mean[0]), vx = mul_(mean[1], ir), vy = mul_(mean[2], ir);
     const Real k2 = mul_(Real(0.5), fma(vx, vx, mul_(vy, vy)));
     const Real p = mul_(gm1, fma(-mean[0], k2, mean[3])), H = mul_(add_(mean[3], p), ir);
     Real c, ic;
-    lengths_(mul_(mul_(gamma, p), ir), c, ic);
+    lim_lengths(mul_(mul_(gamma, p), ir), c, ic);
     const Real b1 = mul_(gm1, mul_(ic, ic)), b2 = mul_(b1, k2);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
