@@ -177,12 +177,16 @@ void launch_chain_stage(rkdg_batch* b, const StageArgs& a, int order) {
                      order == 1 ? b->stream2 : b->stream);
 }
 
-void launch_pack_stage(rkdg_batch* b, const StageArgs& a) {
-    if (!two_chains(b)) return launch_chain_stage(b, a, 0);
-    fork(b);
-    launch_chain_stage(b, a, 2);
-    launch_chain_stage(b, a, 1);
-    join(b);
+// One stage over every tile, n times, with the chains joined at the end as in
+// enqueue_steps.
+void launch_pack_stages(rkdg_batch* b, const StageArgs& a, int n) {
+    const bool two = two_chains(b);
+    if (two) fork(b);
+    for (int i = 0; i < n; ++i) {
+        launch_chain_stage(b, a, two ? 2 : 0);
+        if (two) launch_chain_stage(b, a, 1);
+    }
+    if (two) join(b);
 }
 
 void enqueue_stage(rkdg_batch* b, int order, int s, int in, int u0, int out, bool last) {
@@ -549,9 +553,9 @@ int rkdg_batch_time_stage(rkdg_batch* b, int32_t s, int32_t reps, double* ms) {
         cudaEvent_t e0, e1;
         RKDG_CUDA_TRY(cudaEventCreate(&e0));
         RKDG_CUDA_TRY(cudaEventCreate(&e1));
-        launch_pack_stage(b, a);
+        launch_pack_stages(b, a, 1);
         RKDG_CUDA_TRY(cudaEventRecord(e0, b->stream));
-        for (int i = 0; i < reps; ++i) launch_pack_stage(b, a);
+        launch_pack_stages(b, a, reps);
         RKDG_CUDA_TRY(cudaEventRecord(e1, b->stream));
         RKDG_CUDA_TRY(cudaEventSynchronize(e1));
         float tms = 0;
