@@ -51,8 +51,9 @@ struct rkdg_ctx {
     int pending_out = -1;
     std::unique_ptr<std::ofstream> reslog;  // residual history file (rkdg_set_residual_log)
     bool graph_monitor = false;  // the captured step forms the residual monitor
-    bool resident = false;       // whole steps run in the resident kernel
-    ResidentWork rw;             // its exchange buffers
+    enum { RES_NO, RES_UNTRIED, RES_YES } resident = RES_NO;  // whole steps run in the resident kernel
+    ResidentWork rw;                      // its exchange buffers, from the first step on
+    std::vector<int32_t> halo_entries;    // until then: the tiles' halo lists (TileTables::halo)
 };
 
 namespace {
@@ -227,6 +228,51 @@ void enqueue_step(rkdg_ctx* c, bool monitor) {
     }
 }
 
+// The resident kernel's exchange buffers, in one allocation; false where the
+// device does not hold the solve's tiles at once or has no memory for them.
+bool prepare_resident(rkdg_ctx* c) {
+    const bool lim = c->p.limiter == RKDG_LIMITER_TVB;
+    if (c->tiles.ntiles > resident_tiles(kprec(c), c->p.order, c->p.nq, c->p.flux, lim, c->p.precision == RKDG_FP32C,
+                                         c->tiles.max_halo))
+        return false;
+    const std::vector<int32_t>& halo = c->halo_entries;
+    std::vector<int32_t> slot((size_t)3 * c->ld, -1);
+    for (size_t h = 0; h < halo.size() / 2; ++h) slot[(size_t)halo[2 * h + 1] * c->ld + halo[2 * h]] = (int32_t)h;
+    ResidentWork& w = c->rw;
+    w.slots = std::max(1, (int)(halo.size() / 2));
+    // two parities, two halves per 16-byte row
+    const size_t row = (size_t)4 * 16 * w.slots * (kprec(c) == RKDG_FP64 ? 2 : 1);
+    const size_t trace = row * (c->p.ng + (c->p.flux == RKDG_FLUX_LLF ? 1 : 0)), mean = lim ? row : 0;
+    const size_t zero = trace + mean + kResidentSums, table = sizeof(int32_t) * slot.size();
+    try {
+        w.mem = dev_alloc(c, zero + table);
+    } catch (const Error& e) {
+        if (e.code == RKDG_ERR_NOMEM) return false;
+        throw;
+    }
+    unsigned char* p = static_cast<unsigned char*>(w.mem);
+    w.trace = p;
+    if (lim) w.mean = p + trace;
+    w.sums = p + trace + mean;
+    w.slot = reinterpret_cast<int*>(p + zero);
+    RKDG_CUDA_TRY(cudaMemsetAsync(p, 0, zero, c->stream));
+    w.clean = true;
+    RKDG_CUDA_TRY(cudaMemcpyAsync(w.slot, slot.data(), table, cudaMemcpyHostToDevice, c->stream));
+    (kprec(c) == RKDG_FP64 ? upload_resident_tables_fp64 : upload_resident_tables_fp32)(c->p.nq, c->p.ng);
+    sync(c);  // the host table goes out of scope
+    return true;
+}
+
+// Whether the context's steps run in the resident kernel, decided at its first
+// step: a context that only forms residuals pays for none of it.
+bool use_resident(rkdg_ctx* c) {
+    if (c->resident == rkdg_ctx::RES_UNTRIED) {
+        c->resident = prepare_resident(c) ? rkdg_ctx::RES_YES : rkdg_ctx::RES_NO;
+        c->halo_entries = {};
+    }
+    return c->resident == rkdg_ctx::RES_YES;
+}
+
 // `steps` whole steps (at most kResidentSteps) in one launch, with the state
 // in buffer 0; false: the device does not take the launch, and the context
 // uses the stage kernels from here on
@@ -235,9 +281,10 @@ bool enqueue_resident(rkdg_ctx* c, int steps, bool monitor) {
     StageArgs a = base_args(c);
     a.Unew = c->d.U[0];
     a.far_sid = c->d.far;
-    c->resident = launch_resident(a, c->tiles, c->p.limiter == RKDG_LIMITER_TVB ? c->d.lim : nullptr, c->rw,
-                                  c->p.order, c->p.nq, c->p.flux, kprec(c), c->p.rk, steps, monitor, c->stream);
-    return c->resident;
+    const bool taken = launch_resident(a, c->tiles, c->p.limiter == RKDG_LIMITER_TVB ? c->d.lim : nullptr, c->rw,
+                                       c->p.order, c->p.nq, c->p.flux, kprec(c), c->p.rk, steps, monitor, c->stream);
+    if (!taken) c->resident = rkdg_ctx::RES_NO;
+    return taken;
 }
 
 constexpr int kGraphSteps = 8;
@@ -325,7 +372,7 @@ void destroy_ctx(rkdg_ctx* c) {
     cudaFree(c->d.ctl);
     cudaFree(c->d.far);
     cudaFree(c->d.ref32);
-    for (void* p : {c->rw.trace, c->rw.mean, (void*)c->rw.slot, (void*)c->rw.sums}) cudaFree(p);
+    cudaFree(c->rw.mem);
     cudaFree(c->d.tcode);
     cudaFree(c->d.tdesc);
     cudaFree(c->d.halo);
@@ -487,32 +534,13 @@ int create_ctx(const rkdg_mesh_desc* mesh, const rkdg_params* params, int32_t n_
                 RKDG_CUDA_TRY(cudaMemsetAsync(c->d.tile_flags, 0, nf, c->stream));
                 RKDG_CUDA_TRY(cudaMemsetAsync(c->d.tile_list, 0, nl, c->stream));
             }
-            const bool lim = params->limiter == RKDG_LIMITER_TVB, comp = params->precision == RKDG_FP32C;
-            std::vector<int32_t> slot;
-            if (n_owned < 0 && tt.ntiles <= resident_tiles(kprec(c), params->order, params->nq, params->flux, lim,
-                                                           comp, tt.max_halo)) {
-                c->resident = true;
-                (kprec(c) == RKDG_FP64 ? upload_resident_tables_fp64 : upload_resident_tables_fp32)(params->nq, params->ng);
-                slot.assign((size_t)3 * ld, -1);
-                for (size_t h = 0; h < tt.halo.size() / 2; ++h)
-                    slot[(size_t)tt.halo[2 * h + 1] * ld + tt.halo[2 * h]] = (int32_t)h;
-                ResidentWork& w = c->rw;
-                w.slots = std::max(1, (int)(tt.halo.size() / 2));
-                w.slot = (int*)dev_alloc(c, sizeof(int32_t) * slot.size());
-                RKDG_CUDA_TRY(cudaMemcpyAsync(w.slot, slot.data(), sizeof(int32_t) * slot.size(),
-                                              cudaMemcpyHostToDevice, c->stream));
-                // two parities, two halves per 16-byte row
-                const size_t row = (size_t)4 * 16 * w.slots * (kprec(c) == RKDG_FP64 ? 2 : 1);
-                const size_t nt = row * (params->ng + (params->flux == RKDG_FLUX_LLF ? 1 : 0));
-                w.trace = dev_alloc(c, nt);
-                RKDG_CUDA_TRY(cudaMemsetAsync(w.trace, 0, nt, c->stream));
-                if (lim) {
-                    w.mean = dev_alloc(c, row);
-                    RKDG_CUDA_TRY(cudaMemsetAsync(w.mean, 0, row, c->stream));
-                }
-                w.sums = (unsigned char*)dev_alloc(c, kResidentSums);
-            }
             sync(c);  // host tables go out of scope
+            if (n_owned < 0 && tt.ntiles <= resident_tiles_bound(kprec(c), params->order, params->flux,
+                                                                 params->limiter == RKDG_LIMITER_TVB,
+                                                                 params->precision == RKDG_FP32C, tt.max_halo)) {
+                c->resident = rkdg_ctx::RES_UNTRIED;
+                c->halo_entries = std::move(tt.halo);
+            }
         }
         c->d.partial = (double*)dev_alloc(c, sizeof(double) * 4 * (totals_partial_count(T) + 1));
         c->d.ctl = (StepCtl*)dev_alloc(c, sizeof(StepCtl));
@@ -870,7 +898,7 @@ int rkdg_step(rkdg_ctx* c, double dt, double* dt_used, double* monitor) {
             push_ctl(c);
         }
         c->ctl_fresh = false;
-        if (!c->resident || !enqueue_resident(c, 1, true)) enqueue_step(c, true);
+        if (!use_resident(c) || !enqueue_resident(c, 1, true)) enqueue_step(c, true);
         c->wave_valid = true;
         pull_ctl(c);
         check_error_flag(c);
@@ -899,7 +927,7 @@ int rkdg_advance(rkdg_ctx* c, int32_t nsteps, double t_final, double* t, int32_t
         c->h_ctl->done = 0;
         push_ctl(c);
         c->ctl_fresh = false;
-        if (c->resident) {
+        if (use_resident(c)) {
             int left = nsteps;
             while (left > 0) {
                 const int n = c->reslog ? 1 : std::min(left, kResidentSteps);
@@ -918,7 +946,7 @@ int rkdg_advance(rkdg_ctx* c, int32_t nsteps, double t_final, double* t, int32_t
             if (c->reslog) c->reslog->flush();
             nsteps = left;  // (a refused launch: the rest below)
         }
-        if (c->resident) {
+        if (c->resident == rkdg_ctx::RES_YES) {
             c->wave_valid = true;
             pull_ctl(c);
             check_error_flag(c);

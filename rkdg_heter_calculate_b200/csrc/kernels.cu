@@ -428,6 +428,11 @@ size_t smem_limit() {
     return (size_t)device_attribute(limit, cudaDevAttrMaxSharedMemoryPerBlockOptin) - 1024;
 }
 
+int smem_per_sm() {
+    static PerDevice<int> n;
+    return device_attribute(n, cudaDevAttrMaxSharedMemoryPerMultiprocessor);
+}
+
 int sm_count() {
     static PerDevice<int> n;
     return device_attribute(n, cudaDevAttrMultiProcessorCount);
@@ -587,6 +592,10 @@ void launch_residual(const StageArgs& a, const TileArgs& t, int order, int nq, i
 
 int resident_tiles(int prec, int order, int nq, int flux, bool limiter, bool comp, int max_halo) {
     return (prec == RKDG_FP32 ? resident_tiles_fp32 : resident_tiles_fp64)(order, nq, flux, limiter, comp, max_halo);
+}
+
+int resident_tiles_bound(int prec, int order, int flux, bool limiter, bool comp, int max_halo) {
+    return (prec == RKDG_FP32 ? resident_bound_fp32 : resident_bound_fp64)(order, flux, limiter, comp, max_halo);
 }
 
 bool launch_resident(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,

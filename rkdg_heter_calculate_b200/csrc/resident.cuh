@@ -598,6 +598,11 @@ struct ResidentForm {
             return known[max_halo] = n * sm_count();
         });
     }
+    // no fewer, without a look at the kernels: by shared memory
+    static int bound(int max_halo) {
+        if (max_halo > kTile || SM::bytes(max_halo) > smem_limit()) return 0;
+        return (int)(smem_per_sm() / SM::bytes(max_halo)) * sm_count();
+    }
     static int tiles(int max_halo) { return std::max(fit<256>(max_halo), fit<128>(max_halo)); }
     // 256 threads per tile while the device holds all tiles that way
     // (false: refused as a whole, as under a limit on the SMs a process may use)

@@ -5,6 +5,10 @@ namespace rkdg {
 
 #include "resident.cuh"
 
+int resident_bound_fp32(int order, int flux, bool limiter, bool comp, int max_halo) {
+    return with_resident<float>(order, 6, flux, limiter, comp, [&](auto form) { return form.bound(max_halo); });
+}
+
 int resident_tiles_fp32(int order, int nq, int flux, bool limiter, bool comp, int max_halo) {
     return with_resident<float>(order, nq, flux, limiter, comp, [&](auto form) { return form.tiles(max_halo); });
 }

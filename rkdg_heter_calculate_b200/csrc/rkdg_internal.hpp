@@ -253,6 +253,7 @@ void upload_tables(int nq, int ng);
 // solves of at most resident_tiles(...) tiles (0: none; the tile list's halo
 // lists must fit a CTA) in the locality order, element 0 first.
 struct ResidentWork {            // a context's exchange buffers
+    void* mem = nullptr;         // the one allocation that holds them
     int* slot = nullptr;         // [3][ld] the halo entry (in any tile's list) that reads each element edge, or -1
     int slots = 0;               // halo entries
     void* trace = nullptr;       // [2][rows][2][slots] 16 bytes, zero before the first launch
@@ -264,12 +265,16 @@ struct ResidentWork {            // a context's exchange buffers
 constexpr int kResidentSteps = 64;  // most steps of one launch
 constexpr size_t kResidentSums = kResidentSteps * 12 + 16;
 int resident_tiles(int prec, int order, int nq, int flux, bool limiter, bool comp, int max_halo);
+// no fewer than resident_tiles, from shared memory alone: asking loads no kernel
+int resident_tiles_bound(int prec, int order, int flux, bool limiter, bool comp, int max_halo);
 // its tables (each CUDA translation unit holds its own)
 void upload_resident_tables_fp32(int nq, int ng);
 void upload_resident_tables_fp64(int nq, int ng);
 // (false: the device refused to hold the launch as a whole; nothing was enqueued but the sums' clearing)
 bool launch_resident(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
                      int flux, int prec, int rk, int steps, bool monitor, cudaStream_t stream);
+int resident_bound_fp32(int order, int flux, bool limiter, bool comp, int max_halo);
+int resident_bound_fp64(int order, int flux, bool limiter, bool comp, int max_halo);
 int resident_tiles_fp32(int order, int nq, int flux, bool limiter, bool comp, int max_halo);
 int resident_tiles_fp64(int order, int nq, int flux, bool limiter, bool comp, int max_halo);
 bool launch_resident_fp32(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
@@ -305,6 +310,7 @@ bool tiled_fits(int prec, int order, int flux, int max_halo, int tile);
 int tiled_max_ctas_per_sm(int prec, int order, int nq, int flux, int max_halo, int tile = kTile);
 int current_device();
 int sm_count();       // SMs of the current device
+int smem_per_sm();    // shared memory of an SM, in bytes
 size_t smem_limit();  // dynamic shared memory a CTA may use
 // TVB limiter over tiles; flags[solve] (may be null: all on) enables it per
 // solve, solves whose control block (ctl may be null) says done are skipped,

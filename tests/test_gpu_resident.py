@@ -145,3 +145,20 @@ def test_resident_reports_a_bad_first_time_step(n):
             s.step(float("inf"))
         assert e.value.code == 4
     s.close()
+
+
+def test_exchange_buffers_are_made_at_the_first_step():
+    """A context that only forms residuals does not pay for them; a mesh far too
+    large to be resident never does."""
+    for n, resident in ((20, True), (400, False)):
+        mesh = meshgen.periodic_structured(n, n, jitter=0.15, seed=2)
+        s = CUDARkdgSolver(mesh, farfield=FAR, order=2, nq=6, ng=3, flux="hllc", precision="fp32", cfl=0.2)
+        s.initRKDG()
+        before = s.sizes()[2]
+        s.residual(basis="native")
+        staged = s.sizes()[2]
+        s.advance(3)
+        after = s.sizes()[2]
+        assert staged - before == 0  # (the staging array came with the state)
+        assert after > staged if resident else after == staged
+        s.close()
