@@ -232,8 +232,8 @@ void enqueue_step(rkdg_ctx* c, bool monitor) {
 // device does not hold the solve's tiles at once or has no memory for them.
 bool prepare_resident(rkdg_ctx* c) {
     const bool lim = c->p.limiter == RKDG_LIMITER_TVB;
-    if (c->tiles.ntiles > resident_tiles(kprec(c), c->p.order, c->p.nq, c->p.flux, lim, c->p.precision == RKDG_FP32C,
-                                         c->tiles.max_halo))
+    const ResidentUnit& unit = resident_unit(kprec(c), lim);
+    if (c->tiles.ntiles > unit.tiles(c->p.order, c->p.nq, c->p.flux, c->p.precision == RKDG_FP32C, c->tiles.max_halo))
         return false;
     const std::vector<int32_t>& halo = c->halo_entries;
     std::vector<int32_t> slot((size_t)3 * c->ld, -1);
@@ -258,7 +258,7 @@ bool prepare_resident(rkdg_ctx* c) {
     RKDG_CUDA_TRY(cudaMemsetAsync(p, 0, zero, c->stream));
     w.clean = true;
     RKDG_CUDA_TRY(cudaMemcpyAsync(w.slot, slot.data(), table, cudaMemcpyHostToDevice, c->stream));
-    (kprec(c) == RKDG_FP64 ? upload_resident_tables_fp64 : upload_resident_tables_fp32)(c->p.nq, c->p.ng);
+    unit.upload_tables(c->p.nq, c->p.ng);
     sync(c);  // the host table goes out of scope
     return true;
 }
@@ -281,8 +281,9 @@ bool enqueue_resident(rkdg_ctx* c, int steps, bool monitor) {
     StageArgs a = base_args(c);
     a.Unew = c->d.U[0];
     a.far_sid = c->d.far;
-    const bool taken = launch_resident(a, c->tiles, c->p.limiter == RKDG_LIMITER_TVB ? c->d.lim : nullptr, c->rw,
-                                       c->p.order, c->p.nq, c->p.flux, kprec(c), c->p.rk, steps, monitor, c->stream);
+    const bool lim = c->p.limiter == RKDG_LIMITER_TVB;
+    const bool taken = resident_unit(kprec(c), lim).launch(a, c->tiles, lim ? c->d.lim : nullptr, c->rw, c->p.order,
+                                                           c->p.nq, c->p.flux, c->p.rk, steps, monitor, c->stream);
     if (!taken) c->resident = rkdg_ctx::RES_NO;
     return taken;
 }
@@ -535,9 +536,9 @@ int create_ctx(const rkdg_mesh_desc* mesh, const rkdg_params* params, int32_t n_
                 RKDG_CUDA_TRY(cudaMemsetAsync(c->d.tile_list, 0, nl, c->stream));
             }
             sync(c);  // host tables go out of scope
-            if (n_owned < 0 && tt.ntiles <= resident_tiles_bound(kprec(c), params->order, params->flux,
-                                                                 params->limiter == RKDG_LIMITER_TVB,
-                                                                 params->precision == RKDG_FP32C, tt.max_halo)) {
+            const ResidentUnit& unit = resident_unit(kprec(c), params->limiter == RKDG_LIMITER_TVB);
+            if (n_owned < 0 &&
+                tt.ntiles <= unit.bound(params->order, params->flux, params->precision == RKDG_FP32C, tt.max_halo)) {
                 c->resident = rkdg_ctx::RES_UNTRIED;
                 c->halo_entries = std::move(tt.halo);
             }

@@ -590,20 +590,6 @@ void launch_residual(const StageArgs& a, const TileArgs& t, int order, int nq, i
     dispatch<MODE_RESIDUAL>(a, t, order, nq, flux, prec, ctas, stream);
 }
 
-int resident_tiles(int prec, int order, int nq, int flux, bool limiter, bool comp, int max_halo) {
-    return (prec == RKDG_FP32 ? resident_tiles_fp32 : resident_tiles_fp64)(order, nq, flux, limiter, comp, max_halo);
-}
-
-int resident_tiles_bound(int prec, int order, int flux, bool limiter, bool comp, int max_halo) {
-    return (prec == RKDG_FP32 ? resident_bound_fp32 : resident_bound_fp64)(order, flux, limiter, comp, max_halo);
-}
-
-bool launch_resident(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
-                     int flux, int prec, int rk, int steps, bool monitor, cudaStream_t stream) {
-    return (prec == RKDG_FP32 ? launch_resident_fp32 : launch_resident_fp64)(a, t, lim, w, order, nq, flux, rk, steps, monitor,
-                                                                      stream);
-}
-
 void wait_selftest(double limit_s, int* timed_out, double* waited_s) {
     unsigned long long* d = nullptr;
     RKDG_CUDA_TRY(cudaMalloc(&d, 2 * sizeof(unsigned long long)));

@@ -1,4 +1,4 @@
-// Resident solve kernel (included by kernels.cu): whole time steps of one
+// Resident solve kernel (included by resident_fp*.cu): whole time steps of one
 // solve whose tiles all fit on the device at once, in one cooperative launch.
 //
 // A CTA owns one tile of 128 elements for the launch and keeps its state, U^n
@@ -622,37 +622,29 @@ struct ResidentForm {
 };
 
 // calls f with the form of a method
-template <typename Real0, typename F>
-auto with_resident(int order, int nq, int flux, bool limiter, bool comp, F&& f) {
-    auto lim = [&](auto real, auto nb, auto q, auto g, auto fl, auto l) {
-        using Real = decltype(real);
+template <typename Real, int LIM, typename F>
+auto with_resident(int order, int nq, int flux, bool comp, F&& f) {
+    auto flx = [&](auto nb, auto q, auto g, auto fl) {
         constexpr int NB = decltype(nb)::value, NQ = decltype(q)::value, NG = decltype(g)::value;
-        constexpr int FL = decltype(fl)::value, L = decltype(l)::value;
+        constexpr int FL = decltype(fl)::value;
         if constexpr (sizeof(Real) == 4)
-            if (comp) return f(ResidentForm<Real, NB, NQ, NG, FL, L, 1>{});
-        return f(ResidentForm<Real, NB, NQ, NG, FL, L, 0>{});
+            if (comp) return f(ResidentForm<Real, NB, NQ, NG, FL, LIM, 1>{});
+        return f(ResidentForm<Real, NB, NQ, NG, FL, LIM, 0>{});
     };
-    auto flx = [&](auto real, auto nb, auto q, auto g, auto fl) {
-        if (limiter) return lim(real, nb, q, g, fl, std::integral_constant<int, 1>{});
-        return lim(real, nb, q, g, fl, std::integral_constant<int, 0>{});
+    auto rule = [&](auto nb, auto q, auto g) {
+        if (flux == RKDG_FLUX_HLLC) return flx(nb, q, g, std::integral_constant<int, RKDG_FLUX_HLLC>{});
+        return flx(nb, q, g, std::integral_constant<int, RKDG_FLUX_LLF>{});
     };
-    auto rule = [&](auto real, auto nb, auto q, auto g) {
-        if (flux == RKDG_FLUX_HLLC) return flx(real, nb, q, g, std::integral_constant<int, RKDG_FLUX_HLLC>{});
-        return flx(real, nb, q, g, std::integral_constant<int, RKDG_FLUX_LLF>{});
-    };
-    auto ord = [&](auto real) {
-        using I = std::integral_constant<int, 3>;
-        using S = std::integral_constant<int, 6>;
-        if (order == 1) return rule(real, I{}, I{}, std::integral_constant<int, 2>{});
-        if (nq == 7) return rule(real, S{}, std::integral_constant<int, 7>{}, I{});
-        return rule(real, S{}, S{}, I{});
-    };
-    return ord(Real0(0));
+    using I = std::integral_constant<int, 3>;
+    using S = std::integral_constant<int, 6>;
+    if (order == 1) return rule(I{}, I{}, std::integral_constant<int, 2>{});
+    if (nq == 7) return rule(S{}, std::integral_constant<int, 7>{}, I{});
+    return rule(S{}, S{}, I{});
 }
 
-template <typename Real>
-bool launch_resident_of(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
-                        int flux, int rk, int steps, bool monitor, cudaStream_t stream) {
+template <typename Real, int LIM>
+bool launch_resident(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq, int flux,
+                     int rk, int steps, bool monitor, cudaStream_t stream) {
     ResidentArgs r{};
     r.U = a.Unew;
     r.jinv = a.jinv, r.conn = a.conn, r.lim = lim, r.ctl = a.ctl;
@@ -666,8 +658,21 @@ bool launch_resident_of(const StageArgs& a, const TileArgs& t, const void* lim, 
     w.epoch += (unsigned)(steps * rk);
     if (!w.clean) RKDG_CUDA_TRY(cudaMemsetAsync(w.sums, 0, kResidentSums, stream));
     w.clean = true;  // each launch leaves them so, unless it reports an error
-    return with_resident<Real>(order, nq, flux, lim != nullptr, a.lo_row >= 0,
-                               [&](auto form) { return form.launch(r, t, stream); });
+    return with_resident<Real, LIM>(order, nq, flux, a.lo_row >= 0,
+                                    [&](auto form) { return form.launch(r, t, stream); });
+}
+
+// the unit of a translation unit
+template <typename Real, int LIM>
+constexpr ResidentUnit resident_unit_of() {
+    return ResidentUnit{
+        [](int order, int nq, int flux, bool comp, int max_halo) {
+            return with_resident<Real, LIM>(order, nq, flux, comp, [&](auto form) { return form.tiles(max_halo); });
+        },
+        [](int order, int flux, bool comp, int max_halo) {
+            return with_resident<Real, LIM>(order, 6, flux, comp, [&](auto form) { return form.bound(max_halo); });
+        },
+        upload_module_tables, launch_resident<Real, LIM>};
 }
 
 }  // namespace

@@ -1,23 +1,10 @@
-// The resident solve kernel's FP64 forms (resident.cuh).
+// The resident solve kernel's FP64 forms without the limiter (resident.cuh).
 #include "device.cuh"
 
 namespace rkdg {
 
 #include "resident.cuh"
 
-int resident_bound_fp64(int order, int flux, bool limiter, bool comp, int max_halo) {
-    return with_resident<double>(order, 6, flux, limiter, comp, [&](auto form) { return form.bound(max_halo); });
-}
-
-int resident_tiles_fp64(int order, int nq, int flux, bool limiter, bool comp, int max_halo) {
-    return with_resident<double>(order, nq, flux, limiter, comp, [&](auto form) { return form.tiles(max_halo); });
-}
-
-bool launch_resident_fp64(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
-                          int flux, int rk, int steps, bool monitor, cudaStream_t stream) {
-    return launch_resident_of<double>(a, t, lim, w, order, nq, flux, rk, steps, monitor, stream);
-}
-
-void upload_resident_tables_fp64(int nq, int ng) { upload_module_tables(nq, ng); }
+extern const ResidentUnit resident_fp64 = resident_unit_of<double, 0>();
 
 }  // namespace rkdg

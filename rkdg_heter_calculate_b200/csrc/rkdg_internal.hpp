@@ -250,8 +250,8 @@ inline int state_rows(int precision, int nb) {
 // RKDG_FP32C setting to RKDG_FP32).
 void upload_tables(int nq, int ng);
 // Whole steps of one solve in one cooperative launch (resident.cuh), for
-// solves of at most resident_tiles(...) tiles (0: none; the tile list's halo
-// lists must fit a CTA) in the locality order, element 0 first.
+// solves of at most ResidentUnit::tiles tiles (the tile list's halo lists
+// must fit a CTA) in the locality order, element 0 first.
 struct ResidentWork {            // a context's exchange buffers
     void* mem = nullptr;         // the one allocation that holds them
     int* slot = nullptr;         // [3][ld] the halo entry (in any tile's list) that reads each element edge, or -1
@@ -264,23 +264,25 @@ struct ResidentWork {            // a context's exchange buffers
 };
 constexpr int kResidentSteps = 64;  // most steps of one launch
 constexpr size_t kResidentSums = kResidentSteps * 12 + 16;
-int resident_tiles(int prec, int order, int nq, int flux, bool limiter, bool comp, int max_halo);
-// no fewer than resident_tiles, from shared memory alone: asking loads no kernel
-int resident_tiles_bound(int prec, int order, int flux, bool limiter, bool comp, int max_halo);
-// its tables (each CUDA translation unit holds its own)
-void upload_resident_tables_fp32(int nq, int ng);
-void upload_resident_tables_fp64(int nq, int ng);
-// (false: the device refused to hold the launch as a whole; nothing was enqueued but the sums' clearing)
-bool launch_resident(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
-                     int flux, int prec, int rk, int steps, bool monitor, cudaStream_t stream);
-int resident_bound_fp32(int order, int flux, bool limiter, bool comp, int max_halo);
-int resident_bound_fp64(int order, int flux, bool limiter, bool comp, int max_halo);
-int resident_tiles_fp32(int order, int nq, int flux, bool limiter, bool comp, int max_halo);
-int resident_tiles_fp64(int order, int nq, int flux, bool limiter, bool comp, int max_halo);
-bool launch_resident_fp32(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
-                          int flux, int rk, int steps, bool monitor, cudaStream_t stream);
-bool launch_resident_fp64(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq,
-                          int flux, int rk, int steps, bool monitor, cudaStream_t stream);
+// The resident kernels of an arithmetic, with or without the limiter.  Each
+// is a translation unit of its own (with its own tables): loading the limited
+// FP32 forms takes 5 ms of a process's first step, which solves without the
+// limiter do not pay.
+struct ResidentUnit {
+    // most tiles that the device holds at once (0: none), and a number no
+    // smaller from shared memory alone, for which no kernel is loaded
+    int (*tiles)(int order, int nq, int flux, bool comp, int max_halo);
+    int (*bound)(int order, int flux, bool comp, int max_halo);
+    void (*upload_tables)(int nq, int ng);
+    // (false: the device refused to hold the launch as a whole; nothing was enqueued but the sums' clearing)
+    bool (*launch)(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq, int flux,
+                   int rk, int steps, bool monitor, cudaStream_t stream);
+};
+extern const ResidentUnit resident_fp32, resident_fp32_tvb, resident_fp64, resident_fp64_tvb;
+inline const ResidentUnit& resident_unit(int prec, bool limiter) {
+    if (prec == RKDG_FP32) return limiter ? resident_fp32_tvb : resident_fp32;
+    return limiter ? resident_fp64_tvb : resident_fp64;
+}
 // The tile-staged stage kernel: one CTA per tile of kTile elements (each
 // interior flux once per tile, traces shared in shared memory), `ctas` CTAs
 // per launch looping over the tiles (0 = one CTA per tile).  `order` 1 or 2,
