@@ -12,6 +12,7 @@
 #include <string>
 #include <vector>
 
+#include "per_device.hpp"
 #include "rkdg_internal.hpp"
 
 namespace rkdg {
@@ -52,6 +53,7 @@ struct rkdg_ctx {
     std::unique_ptr<std::ofstream> reslog;  // residual history file (rkdg_set_residual_log)
     bool graph_monitor = false;  // the captured step forms the residual monitor
     enum { RES_NO, RES_UNTRIED, RES_YES } resident = RES_NO;  // whole steps run in the resident kernel
+    int res_tiles[2] = {0, 0};            // tiles that fit on the device with 128 and with 256 threads each
     ResidentWork rw;                      // its exchange buffers, from the first step on
     std::vector<int32_t> halo_entries;    // until then: the tiles' halo lists (TileTables::halo)
 };
@@ -233,8 +235,10 @@ void enqueue_step(rkdg_ctx* c, bool monitor) {
 bool prepare_resident(rkdg_ctx* c) {
     const bool lim = c->p.limiter == RKDG_LIMITER_TVB;
     const ResidentUnit& unit = resident_unit(kprec(c), lim);
-    if (c->tiles.ntiles > unit.tiles(c->p.order, c->p.nq, c->p.flux, c->p.precision == RKDG_FP32C, c->tiles.max_halo))
-        return false;
+    for (int wide = 0; wide < 2; ++wide)
+        c->res_tiles[wide] = unit.tiles(c->p.order, c->p.nq, c->p.flux, c->p.precision == RKDG_FP32C,
+                                        c->tiles.max_halo, wide != 0);
+    if (c->tiles.ntiles > std::max(c->res_tiles[0], c->res_tiles[1])) return false;
     const std::vector<int32_t>& halo = c->halo_entries;
     std::vector<int32_t> slot((size_t)3 * c->ld, -1);
     for (size_t h = 0; h < halo.size() / 2; ++h) slot[(size_t)halo[2 * h + 1] * c->ld + halo[2 * h]] = (int32_t)h;
@@ -273,17 +277,62 @@ bool use_resident(rkdg_ctx* c) {
     return c->resident == rkdg_ctx::RES_YES;
 }
 
+// What the step calls in flight (rkdg_step, rkdg_advance, of any thread) take of
+// each device, in millionths: a context's tiles of those it holds at once.
+PerDevice<int64_t> g_load;
+
+// The form a step call runs in, chosen by what the device has left, and its
+// share of it for as long as the call lasts.  Resident launches are held whole
+// or not at all, so beyond one device of them they queue, each at one solve's
+// latency, while stage launches of several solves fill the device together:
+// 8 threads with 20,000 P1 FP32 triangles each, 100 steps, 9.2 ms all resident,
+// 3.3 as chosen here (one alone: 1.0; 1.9 through the stage kernels), P2 11.0
+// and 5.1, FP64 with the limiter 19.4 and 9.2.  So: 256 threads per tile while
+// that fits beside the others, then 128, then the stage kernels (the same
+// bits).
+class StepShare {
+public:
+    enum Form { STAGES, NARROW, WIDE };
+    explicit StepShare(rkdg_ctx* c) : device_(c->device) {
+        const bool resident = use_resident(c);
+        auto part = [&](int wide) {  // (a mesh that is never resident: the whole device)
+            const int64_t n = c->tiles.ntiles, fit = resident ? c->res_tiles[wide] : 0;
+            return fit >= n ? (n * kDevice + fit - 1) / fit : kDevice;
+        };
+        const int64_t narrow = part(0), wide = part(1);
+        g_load.use(device_, [&](int64_t& load) {
+            if (resident && c->tiles.ntiles <= c->res_tiles[1] && load + wide <= kDevice) form_ = WIDE, share_ = wide;
+            else if (resident && c->tiles.ntiles <= c->res_tiles[0] && load + narrow <= kDevice) form_ = NARROW, share_ = narrow;
+            else share_ = std::min(narrow, wide);
+            load += share_;
+        });
+    }
+    ~StepShare() {
+        g_load.use(device_, [&](int64_t& load) { load -= share_; });
+    }
+    StepShare(const StepShare&) = delete;
+    StepShare& operator=(const StepShare&) = delete;
+    Form form() const { return form_; }
+
+private:
+    static constexpr int64_t kDevice = 1000000;
+    int device_;
+    Form form_ = STAGES;
+    int64_t share_ = 0;
+};
+
 // `steps` whole steps (at most kResidentSteps) in one launch, with the state
 // in buffer 0; false: the device does not take the launch, and the context
 // uses the stage kernels from here on
-bool enqueue_resident(rkdg_ctx* c, int steps, bool monitor) {
+bool enqueue_resident(rkdg_ctx* c, int steps, bool monitor, StepShare::Form form) {
     c->ctl_fresh = false;
     StageArgs a = base_args(c);
     a.Unew = c->d.U[0];
     a.far_sid = c->d.far;
     const bool lim = c->p.limiter == RKDG_LIMITER_TVB;
     const bool taken = resident_unit(kprec(c), lim).launch(a, c->tiles, lim ? c->d.lim : nullptr, c->rw, c->p.order,
-                                                           c->p.nq, c->p.flux, c->p.rk, steps, monitor, c->stream);
+                                                           c->p.nq, c->p.flux, c->p.rk, steps, monitor, form == StepShare::WIDE,
+                                                           c->stream);
     if (!taken) c->resident = rkdg_ctx::RES_NO;
     return taken;
 }
@@ -899,7 +948,8 @@ int rkdg_step(rkdg_ctx* c, double dt, double* dt_used, double* monitor) {
             push_ctl(c);
         }
         c->ctl_fresh = false;
-        if (!use_resident(c) || !enqueue_resident(c, 1, true)) enqueue_step(c, true);
+        const StepShare share(c);
+        if (share.form() == StepShare::STAGES || !enqueue_resident(c, 1, true, share.form())) enqueue_step(c, true);
         c->wave_valid = true;
         pull_ctl(c);
         check_error_flag(c);
@@ -928,12 +978,15 @@ int rkdg_advance(rkdg_ctx* c, int32_t nsteps, double t_final, double* t, int32_t
         c->h_ctl->done = 0;
         push_ctl(c);
         c->ctl_fresh = false;
-        if (use_resident(c)) {
+        const StepShare share(c);
+        bool resident = share.form() != StepShare::STAGES;
+        if (resident) {
             int left = nsteps;
             while (left > 0) {
                 const int n = c->reslog ? 1 : std::min(left, kResidentSteps);
                 const int before = c->h_ctl->step;
-                if (!enqueue_resident(c, n, (bool)c->reslog)) break;
+                resident = enqueue_resident(c, n, (bool)c->reslog, share.form());
+                if (!resident) break;
                 left -= n;
                 // with a final time, stop once the device says done; the
                 // history needs every step's monitor
@@ -947,7 +1000,7 @@ int rkdg_advance(rkdg_ctx* c, int32_t nsteps, double t_final, double* t, int32_t
             if (c->reslog) c->reslog->flush();
             nsteps = left;  // (a refused launch: the rest below)
         }
-        if (c->resident == rkdg_ctx::RES_YES) {
+        if (resident) {
             c->wave_valid = true;
             pull_ctl(c);
             check_error_flag(c);

@@ -603,12 +603,12 @@ struct ResidentForm {
         if (max_halo > kTile || SM::bytes(max_halo) > smem_limit()) return 0;
         return (int)(smem_per_sm() / SM::bytes(max_halo)) * sm_count();
     }
-    static int tiles(int max_halo) { return std::max(fit<256>(max_halo), fit<128>(max_halo)); }
-    // 256 threads per tile while the device holds all tiles that way
+    static int tiles(int max_halo, bool wide) { return wide ? fit<256>(max_halo) : fit<128>(max_halo); }
+    // with 256 threads per tile (wide) or 128
     // (false: refused as a whole, as under a limit on the SMs a process may use)
-    static bool launch(ResidentArgs a, TileArgs t, cudaStream_t s) {
+    static bool launch(ResidentArgs a, TileArgs t, bool wide, cudaStream_t s) {
         void* args[] = {&a, &t};
-        const bool wide = t.ntiles <= fit<256>(t.max_halo);
+        tiles(t.max_halo, wide);  // (sets the kernel's attributes)
         const void* k = wide ? (const void*)kernel<256>() : (const void*)kernel<128>();
         const cudaError_t e = cudaLaunchCooperativeKernel(k, dim3(t.ntiles), dim3(wide ? 256 : 128), args,
                                                           SM::bytes(t.max_halo), s);
@@ -644,7 +644,7 @@ auto with_resident(int order, int nq, int flux, bool comp, F&& f) {
 
 template <typename Real, int LIM>
 bool launch_resident(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq, int flux,
-                     int rk, int steps, bool monitor, cudaStream_t stream) {
+                     int rk, int steps, bool monitor, bool wide, cudaStream_t stream) {
     ResidentArgs r{};
     r.U = a.Unew;
     r.jinv = a.jinv, r.conn = a.conn, r.lim = lim, r.ctl = a.ctl;
@@ -659,15 +659,15 @@ bool launch_resident(const StageArgs& a, const TileArgs& t, const void* lim, Res
     if (!w.clean) RKDG_CUDA_TRY(cudaMemsetAsync(w.sums, 0, kResidentSums, stream));
     w.clean = true;  // each launch leaves them so, unless it reports an error
     return with_resident<Real, LIM>(order, nq, flux, a.lo_row >= 0,
-                                    [&](auto form) { return form.launch(r, t, stream); });
+                                    [&](auto form) { return form.launch(r, t, wide, stream); });
 }
 
 // the unit of a translation unit
 template <typename Real, int LIM>
 constexpr ResidentUnit resident_unit_of() {
     return ResidentUnit{
-        [](int order, int nq, int flux, bool comp, int max_halo) {
-            return with_resident<Real, LIM>(order, nq, flux, comp, [&](auto form) { return form.tiles(max_halo); });
+        [](int order, int nq, int flux, bool comp, int max_halo, bool wide) {
+            return with_resident<Real, LIM>(order, nq, flux, comp, [&](auto form) { return form.tiles(max_halo, wide); });
         },
         [](int order, int flux, bool comp, int max_halo) {
             return with_resident<Real, LIM>(order, 6, flux, comp, [&](auto form) { return form.bound(max_halo); });

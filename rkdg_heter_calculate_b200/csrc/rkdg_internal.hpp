@@ -269,14 +269,15 @@ constexpr size_t kResidentSums = kResidentSteps * 12 + 16;
 // FP32 forms takes 5 ms of a process's first step, which solves without the
 // limiter do not pay.
 struct ResidentUnit {
-    // most tiles that the device holds at once (0: none), and a number no
-    // smaller from shared memory alone, for which no kernel is loaded
-    int (*tiles)(int order, int nq, int flux, bool comp, int max_halo);
+    // most tiles that the device holds at once (0: none) with 256 threads each
+    // (wide) or 128, and a number no smaller from shared memory alone, for
+    // which no kernel is loaded
+    int (*tiles)(int order, int nq, int flux, bool comp, int max_halo, bool wide);
     int (*bound)(int order, int flux, bool comp, int max_halo);
     void (*upload_tables)(int nq, int ng);
     // (false: the device refused to hold the launch as a whole; nothing was enqueued but the sums' clearing)
     bool (*launch)(const StageArgs& a, const TileArgs& t, const void* lim, ResidentWork& w, int order, int nq, int flux,
-                   int rk, int steps, bool monitor, cudaStream_t stream);
+                   int rk, int steps, bool monitor, bool wide, cudaStream_t stream);
 };
 extern const ResidentUnit resident_fp32, resident_fp32_tvb, resident_fp64, resident_fp64_tvb;
 inline const ResidentUnit& resident_unit(int prec, bool limiter) {

@@ -61,7 +61,7 @@ void run() {
     TileArgs t{};
     t.code = up(code), t.desc = up(desc), t.halo = up(halo), t.task = up(task), t.max_halo = 8, t.ntiles = 1;
     using Form = ResidentForm<double, 3, 3, 2, RKDG_FLUX_HLLC, 1, 0>;
-    Form::tiles(t.max_halo);  // sets the kernels' attributes
+    Form::fit<128>(t.max_halo);  // sets the kernels' attributes
     for (int launch = 0; launch < 2; ++launch) {
         void* args[] = {&a, &t};
         const auto t0 = std::chrono::steady_clock::now();
