@@ -3,7 +3,8 @@
 // a neighbour's mean that nobody publishes in the first stage of a step and
 // that lies ready in the second: the wait for it runs out after its two
 // seconds.  Prints the error word, the done flag, the steps and the
-// milliseconds of that launch and of a second one behind it.
+// milliseconds of that launch and of a second one behind it, then whether a
+// launch of more tiles than the device holds is refused, and the error it leaves.
 #include <chrono>
 #include <cstdio>
 #include <cstring>
@@ -73,6 +74,9 @@ void run() {
         std::printf("%d %d %d %.0f\n", c.error, c.done, c.step, ms);
         a.epoch += 2;
     }
+    t.ntiles = 1 << 20;
+    const bool refused = !Form::launch(a, t, false, 0);
+    std::printf("%d %d\n", refused, (int)cudaPeekAtLastError());
 }
 }  // namespace rkdg
 

@@ -226,3 +226,17 @@ def test_solves_in_several_threads_share_the_device(precision, order, flux):
     for s in solvers:
         s.close()
     assert eight < 6.5 * one, (eight, one)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32", "fp32c"])
+@pytest.mark.parametrize("order,nq,flux,limiter,rk", [(1, 3, "hllc", "tvb", 3), (1, 3, "llf", "tvb", 2),
+                                                      (2, 7, "llf", None, 3), (2, 6, "llf", "tvb", 3),
+                                                      (2, 6, "hllc", "tvb", 3), (1, 3, "llf", None, 3)])
+def test_resident_with_128_threads_per_tile(precision, order, nq, flux, limiter, rk):
+    """Meshes that the device holds only with 128 threads per tile: beyond one
+    (FP64) and two (FP32) tiles of 256 threads per SM."""
+    kw = dict(order=order, nq=nq, ng=2 if order == 1 else 3, flux=flux, limiter=limiter, rk=rk, precision=precision,
+              cfl=0.15)
+    for nx, ny in ((160, 60), (190, 99)) if precision == "fp64" else ((200, 96), (270, 139)):
+        mesh = ordered(meshgen.channel(nx, ny))  # 150, 294; 300 and 587 tiles
+        both(mesh, start(mesh, 3 if order == 1 else 6, (1.4, 4.2, 0.0, 8.8), "jump"), (1.4, 4.2, 0.0, 8.8), 4, **kw)

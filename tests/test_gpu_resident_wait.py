@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.fixture(scope="module")
 def launches(tmp_path_factory):
-    """(error word, done, steps, ms) after each of two queued launches."""
+    """(error word, done, steps, ms) after each of two queued launches, and
+    (refused, last error) of one too large for the device."""
     here = os.path.dirname(os.path.abspath(__file__))
     exe = str(tmp_path_factory.mktemp("wait") / "resident_wait")
     subprocess.run([build.nvcc(), "-O3", "-std=c++17", "-I", build.INCLUDE, "-I", build.CSRC,
@@ -31,5 +32,10 @@ def test_a_lost_mean_is_reported(launches):
 def test_launches_behind_a_lost_wait_leave_at_once(launches):
     """A whole advance is queued without a read-back in between: none of the
     launches behind the failed one may wait again, or step on from its state."""
-    (_, done, steps, _), (error, _, steps2, ms) = launches
+    (_, done, steps, _), (error, _, steps2, ms) = launches[:2]
     assert done == 1 and steps == steps2 == 0 and error == 2 and ms < 500, launches
+
+
+def test_a_launch_too_large_is_refused_without_an_error(launches):
+    """The caller falls back to the stage kernels."""
+    assert launches[2] == (1, 0)
