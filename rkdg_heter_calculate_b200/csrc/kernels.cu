@@ -458,15 +458,14 @@ void launch_dependent(bool early, void (*kernel)(P...), int grid, int block, siz
     RKDG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
 }
 
-// Shared-memory attributes of one instantiation for a halo size; returns the
-// dynamic shared memory per CTA.
-
 // The stage kernel of an arithmetic type.
 template <typename Real, int NQ2, int FLUX, int MODE, int ORD, int BT, int LAT = 0>
 constexpr auto stage_kernel() {
     if constexpr (sizeof(Real) == 8) return &stage_fp64_kernel<NQ2, FLUX, MODE, ORD, BT, LAT>;
     else return &tiled_stage_kernel<NQ2, FLUX, MODE, ORD, BT>;
 }
+// Shared-memory attributes of one instantiation for a halo size; returns the
+// dynamic shared memory per CTA.
 template <typename Real, int NQ2, int FLUX, int MODE, int ORD, int BT, int LAT = 0>
 size_t prepare_tiled(int max_halo) {
     const size_t smem = TiledSmem<Real, ORD, FLUX, BT>::bytes(max_halo);
@@ -514,9 +513,14 @@ void launch_tiled(const StageArgs& a, const TileArgs& t, int ctas, cudaStream_t 
     // FP32 kernels prefetch a device of CTAs ahead (prefetch_ahead).  Below 7/8
     // of such a device they start only after the launch before: CTAs that start
     // early fill the free places of some SMs, and a stage of less than one wave
-    // then runs unevenly spread (FP32C P2, 565 tiles of 888: 38.8 us a step
-    // against 32.3; from 792 tiles on 40.3 against 41.6).  FP64 gains at every
-    // size (352 to 3,907 tiles: 1-4 %).
+    // then runs unevenly spread.  Every form measured crosses over at 0.8 to
+    // 0.9 of its device (us per step, early against after):
+    //   P2 HLLC, 888 places   703 tiles 37.1, 35.3   784 tiles 36.8, 37.5
+    //   P2 LLF FP32C          589 tiles 34.4, 31.8   644 tiles 34.7, 36.2
+    //   P2 LLF limited        757 tiles 50.8, 51.0   886 tiles 52.2, 53.8
+    //   P1 HLLC, 1184 places  1001 tiles 27.7, 27.3  1041 tiles 27.9, 28.7
+    //   P1 LLF limited        1001 tiles 37.2, 35.6  1098 tiles 37.2, 38.5
+    // FP64 gains at every size (352 to 3,907 tiles: 1-4 %).
     bool early = true;
     if constexpr (sizeof(Real) == 4) {
         const int device = sm_count() * occupancy_tiled<Real, NQ2, FLUX, MODE, ORD, BT>(t.max_halo);

@@ -42,7 +42,7 @@ struct ResidentArgs {
     double gamma, tvb_m;
     const double* far;   // [4]
     const float* ref32;  // [8]
-    int ld, rk, nsteps, monitor, lo_row;
+    int ld, rk, nsteps, monitor;
     const int* slot;     // [3][ld] the slot each element edge is published in (-1: none)
     int slots;           // one per halo entry, in the order of the tiles' halo lists
     ulonglong2* trace;   // [2][rows][2][slots] the exchanged traces and means (LLF)
@@ -649,7 +649,7 @@ bool launch_resident(const StageArgs& a, const TileArgs& t, const void* lim, Res
     r.U = a.Unew;
     r.jinv = a.jinv, r.conn = a.conn, r.lim = lim, r.ctl = a.ctl;
     r.gamma = a.gamma, r.tvb_m = a.tvb_m, r.far = a.far_sid, r.ref32 = a.ref32;
-    r.ld = a.ld, r.rk = rk, r.nsteps = steps, r.monitor = monitor ? 1 : 0, r.lo_row = a.lo_row;
+    r.ld = a.ld, r.rk = rk, r.nsteps = steps, r.monitor = monitor ? 1 : 0;
     r.slot = w.slot, r.slots = w.slots;
     r.trace = static_cast<ulonglong2*>(w.trace), r.mean = static_cast<ulonglong2*>(w.mean), r.epoch = w.epoch;
     r.wave = reinterpret_cast<unsigned long long*>(w.sums);

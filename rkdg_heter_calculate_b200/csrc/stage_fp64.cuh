@@ -1,4 +1,4 @@
-// FP64 form of the tile-staged stage kernel (included by kernels.cu after
+// FP64 form of the tile-staged stage kernel (included by device.cuh after
 // stage_tiled.cuh, whose staging pipeline, tile tables and shared-memory
 // areas it shares): one thread per element.
 //

@@ -1,4 +1,4 @@
-// Tile-staged fused stage kernel (included by kernels.cu): the staging
+// Tile-staged fused stage kernel (included by device.cuh): the staging
 // pipeline and the FP32 kernel (FP64: stage_fp64.cuh).
 //
 // A tile is up to BT consecutive (locality-ordered) elements of one
