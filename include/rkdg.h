@@ -356,8 +356,9 @@ int rkdg_batch_set_shape(rkdg_batch* b, int32_t ctas, int32_t tile_order);
  * result does not depend on the tile size beyond rounding (interface
  * fluxes are formed once per tile pair). */
 int rkdg_batch_set_tile(rkdg_batch* b, int32_t tile);
-/* Mean device milliseconds of one launch of stage s over all solves (the
- * last stage with its CFL and monitor epilogue, as it runs in a step). */
+/* Mean device milliseconds of stage s over all solves (the last stage with its
+ * CFL and monitor epilogue, as it runs in a step); in tile order 2 the two
+ * orders' launches run side by side over all the repetitions, as in a step. */
 int rkdg_batch_time_stage(rkdg_batch* b, int32_t s, int32_t reps, double* ms_per_launch);
 int rkdg_batch_get_sizes(const rkdg_batch* b, int64_t* elements, int32_t* ntiles, size_t* device_bytes);
 int rkdg_batch_get_stream(const rkdg_batch* b, void** stream);

@@ -29,7 +29,7 @@
 // issues the copies, the reference state comes from a table, and the edge
 // tables are loaded once per CTA: 980,000 P2 triangles 0.288 -> 0.263 ms per
 // step in FP32 and 0.310 -> 0.289 in FP32C, P1 with LLF 0.171 -> 0.158; with
-// overlapping launches and branch-free flux stores 0.254, 0.277 and 0.148.
+// overlapping launches and branch-free flux stores 0.254, 0.276 and 0.148.
 //
 // Staging pipeline: a tile's own state rows are contiguous 16-byte rows in
 // HBM (pack p of element e at (p ld + e) 16), so one thread moves them into
