@@ -14,6 +14,7 @@
 #include <string>
 #include <vector>
 
+#include "device_load.hpp"
 #include "rkdg_internal.hpp"
 
 using namespace rkdg;
@@ -536,6 +537,8 @@ int rkdg_batch_advance(rkdg_batch* b, int32_t nsteps, const double* t_final, dou
             b->h_ctl[s].done = 0;
         }
         push(b);
+        const int per_sm = tiled_max_ctas_per_sm(kprec(b), b->ord, b->p.nq, b->p.flux, b->max_halo, b->tile);
+        const LoadShare share(b->device, stage_share(b->ntiles, (int64_t)per_sm * sm_count()));
         if (!b->graph) b->graph = capture_steps(b, 1);
         if (!b->graph_n && nsteps >= kGraphSteps) b->graph_n = capture_steps(b, kGraphSteps);
         int left = nsteps;

@@ -12,7 +12,7 @@
 #include <string>
 #include <vector>
 
-#include "per_device.hpp"
+#include "device_load.hpp"
 #include "rkdg_internal.hpp"
 
 namespace rkdg {
@@ -22,6 +22,11 @@ thread_local std::string g_last_error;
 }
 
 void set_error(const std::string& msg) { g_last_error = msg; }
+
+PerDevice<int64_t>& device_load() {
+    static PerDevice<int64_t> load;
+    return load;
+}
 
 }  // namespace rkdg
 
@@ -277,48 +282,43 @@ bool use_resident(rkdg_ctx* c) {
     return c->resident == rkdg_ctx::RES_YES;
 }
 
-// What the step calls in flight (rkdg_step, rkdg_advance, of any thread) take of
-// each device, in millionths: a context's tiles of those it holds at once.
-PerDevice<int64_t> g_load;
-
-// The form a step call runs in, chosen by what the device has left, and its
-// share of it for as long as the call lasts.  Resident launches are held whole
-// or not at all, so beyond one device of them they queue, each at one solve's
-// latency, while stage launches of several solves fill the device together:
+// The form a step call runs in, chosen by what the calls in flight leave of the
+// device.  Resident launches are held whole or not at all and keep their places
+// while they wait for one another's tiles: beyond one device of them they
+// queue, each at one solve's latency, and stage launches beside them get what
+// is left, while stage launches of several solves fill the device together.
 // 8 threads with 20,000 P1 FP32 triangles each, 100 steps, 9.2 ms all resident,
 // 3.3 as chosen here (one alone: 1.0; 1.9 through the stage kernels), P2 11.0
-// and 5.1, FP64 with the limiter 19.4 and 9.2.  So: 256 threads per tile while
-// that fits beside the others, then 128, then the stage kernels (the same
-// bits).
+// and 5.1, FP64 with the limiter 19.4 and 9.2; 500,000 triangles beside a
+// resident loop of 33,800 step 3.7 times slower than beside its stage kernels.
+// So: 256 threads per tile while that fits beside the others, then 128, then
+// the stage kernels (the same bits).
 class StepShare {
 public:
     enum Form { STAGES, NARROW, WIDE };
-    explicit StepShare(rkdg_ctx* c) : device_(c->device) {
-        const bool resident = use_resident(c);
-        auto part = [&](int wide) {  // (a mesh that is never resident: the whole device)
-            const int64_t n = c->tiles.ntiles, fit = resident ? c->res_tiles[wide] : 0;
-            return fit >= n ? (n * kDevice + fit - 1) / fit : kDevice;
+    explicit StepShare(rkdg_ctx* c) : load_(c->device) {
+        const int64_t n = c->tiles.ntiles;
+        if (!use_resident(c)) {
+            const int per_sm = tiled_max_ctas_per_sm(kprec(c), c->p.order, c->p.nq, c->p.flux, c->tiles.max_halo);
+            load_.take([&](int64_t) { return stage_share(n, (int64_t)per_sm * sm_count()); });
+            return;
+        }
+        auto part = [&](int wide) {
+            const int64_t fit = c->res_tiles[wide];
+            return fit >= n ? (n * kWholeDevice + fit - 1) / fit : kWholeDevice + 1;
         };
         const int64_t narrow = part(0), wide = part(1);
-        g_load.use(device_, [&](int64_t& load) {
-            if (resident && c->tiles.ntiles <= c->res_tiles[1] && load + wide <= kDevice) form_ = WIDE, share_ = wide;
-            else if (resident && c->tiles.ntiles <= c->res_tiles[0] && load + narrow <= kDevice) form_ = NARROW, share_ = narrow;
-            else share_ = std::min(narrow, wide);
-            load += share_;
+        load_.take([&](int64_t load) {
+            if (load + wide <= kWholeDevice) return form_ = WIDE, wide;
+            if (load + narrow <= kWholeDevice) return form_ = NARROW, narrow;
+            return std::min(narrow, wide);
         });
     }
-    ~StepShare() {
-        g_load.use(device_, [&](int64_t& load) { load -= share_; });
-    }
-    StepShare(const StepShare&) = delete;
-    StepShare& operator=(const StepShare&) = delete;
     Form form() const { return form_; }
 
 private:
-    static constexpr int64_t kDevice = 1000000;
-    int device_;
+    LoadShare load_;
     Form form_ = STAGES;
-    int64_t share_ = 0;
 };
 
 // `steps` whole steps (at most kResidentSteps) in one launch, with the state

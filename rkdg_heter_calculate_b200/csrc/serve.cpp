@@ -26,6 +26,7 @@
 #include <thread>
 #include <vector>
 
+#include "device_load.hpp"
 #include "rkdg_internal.hpp"
 
 using namespace rkdg;
@@ -470,6 +471,9 @@ void engine_loop(rkdg_server* s) {
                 if (s->fault_after == 0) throw Error{RKDG_ERR_CUDA, "engine stopped by rkdg_server_inject_fault"};
                 if (s->fault_after > 0) --s->fault_after;
             }
+            int64_t part = 0;
+            for (int l = 0; l < kLists; ++l) part += stage_share(s->ntiles[l], s->ctas[l]);
+            const LoadShare share(s->device, std::min(part, kWholeDevice));
             const double t0 = now_s();
             RKDG_CUDA_TRY(cudaGraphLaunch(s->graph, s->stream));
             RKDG_CUDA_TRY(cudaMemcpyAsync(s->h_ctl, s->ctl, sizeof(StepCtl) * s->max_slots,
